@@ -9,14 +9,19 @@
 // the string (Python simulate_nfa). Outputs: the final mask and accept flag
 // (s & accept_mask != 0; a rejected string has the empty mask).
 //
-// Design: "four Russians" tables. For every symbol c the 64 source bits are
-// cut into groups of B bits and tbl[c][g][v] holds the OR of the columns of
-// the set bits of v, so a step is ceil(64/B) table lookups ORed together.
-// Symbol index sigma is an extra table: the identity (skip) or all zeros
-// (reject), so bytes >= sigma need no branch. B is picked so all tables fit
-// in shared memory: the widest of 8, 7, 6, 5, 4 bits that fits (8 lookups a
-// byte for sigma <= 12, 10 for sigma <= 21, 11 for sigma <= 39); larger
-// alphabets read 8-bit tables (8 lookups) from global memory through L1.
+// Design: "four Russians" tables. For every symbol c the T source bits are
+// cut into G groups of nearly equal width (T mod G of them one bit wider) and
+// tbl[c][g][v] holds the OR of the columns of the set bits of v, so a step is G
+// table lookups ORed together. Symbol index sigma is an extra table: the
+// identity (skip) or all zeros (reject), so bytes >= sigma need no branch.
+// T = 64, or 32 / 16 for automata of that many states, whose masks and entries
+// are 32-bit words. G is the smallest number of groups (of at most 8 bits) whose
+// tables fit in shared memory: a step is bound by the shared-memory wavefronts
+// of its lookups (about five a warp lookup of random 64-bit entries), so each
+// group less is that share of the time. 64 states, 20 symbols: 9 groups (one of
+// 8 bits, eight of 7) take the memory that ten 7-bit groups took: 262144 strings of
+// 4096 bytes 5.83 -> 5.37 ms (184 -> 200 Gchar/s). Larger alphabets than fit at 16
+// groups read 8-bit tables from global memory through L1.
 // One persistent CTA per SM, a thread per string; threads take strings from
 // an atomic counter and walk them in 16-byte windows.
 #include <algorithm>
@@ -31,19 +36,33 @@ namespace trex {
 constexpr int kNfaThreads = 1024;
 constexpr size_t kNfaSmemBudget = 220 * 1024;
 
-__host__ __device__ constexpr int nfa_groups(int B) { return (64 + B - 1) / B; }
+// Group g of T bits in G groups: width, first bit, first table entry.
+__host__ __device__ constexpr int nfa_width(int T, int G, int g) { return T / G + (g < T % G ? 1 : 0); }
+__host__ __device__ constexpr int nfa_shift(int T, int G, int g) { return g * (T / G) + (g < T % G ? g : T % G); }
+__host__ __device__ constexpr int nfa_first(int T, int G, int g) {
+    int e = 0;
+    for (int k = 0; k < g; ++k) e += 1 << nfa_width(T, G, k);
+    return e;
+}
+__host__ __device__ constexpr int nfa_table_entries(int T, int G) { return nfa_first(T, G, G); }
 // Entries of symbol c are stored at v ^ swizzle(c): with dense states many
 // lanes look up the same v for different symbols, and every table starts on
-// the same bank; the XOR sends them to different bank pairs.
-__host__ __device__ constexpr uint32_t nfa_swizzle(uint32_t c) { return (c ^ (c >> 4)) & 15u; }
-__host__ __device__ constexpr int nfa_table_entries(int B) { return nfa_groups(B) << B; }
+// the same bank; the XOR sends them to different banks (pairs of 64-bit entries).
+template <int T>
+__host__ __device__ constexpr uint32_t nfa_swizzle(uint32_t c) {
+    return T > 32 ? (c ^ (c >> 4)) & 15u : (c ^ (c >> 5)) & 31u;
+}
+// Masks and table entries of T states.
+template <int T> struct NfaWord { using type = uint64_t; };
+template <> struct NfaWord<32> { using type = uint32_t; };
+template <> struct NfaWord<16> { using type = uint32_t; };
 
 struct NfaParams {
     const uint8_t *data;
     int64_t total_bytes;
     const int64_t *offsets;
     int64_t n;
-    const uint64_t *tables;   // (sigma + 1) x groups x 2^B
+    const void *tables;       // (sigma + 1) x entries of the layout
     int sigma;
     uint64_t start_mask, accept_mask;
     uint64_t *final_mask;
@@ -53,27 +72,26 @@ struct NfaParams {
     uint32_t *err;
 };
 
-template <int B>
-__device__ __forceinline__ uint64_t nfa_step(const uint64_t *tbl, uint64_t s, uint32_t byte,
-                                             int sigma) {
-    constexpr int G = nfa_groups(B);
-    constexpr uint32_t MASK = (1u << B) - 1u;
+template <int T, int G>
+__device__ __forceinline__ typename NfaWord<T>::type nfa_step(const typename NfaWord<T>::type *tbl,
+                                                              typename NfaWord<T>::type s, uint32_t byte,
+                                                              int sigma) {
     const uint32_t sym = min(byte, (uint32_t)sigma);
-    const uint64_t *t = tbl + (size_t)sym * nfa_table_entries(B);
-    const uint32_t x = nfa_swizzle(sym) & MASK;
-    uint64_t acc = 0;
+    const typename NfaWord<T>::type *t = tbl + (size_t)sym * nfa_table_entries(T, G);
+    const uint32_t x = nfa_swizzle<T>(sym);
+    typename NfaWord<T>::type acc = 0;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        const uint32_t v = ((uint32_t)(s >> (B * g)) & MASK) ^ x;
-        acc |= t[(g << B) + v];
+        const uint32_t m = (1u << nfa_width(T, G, g)) - 1u;
+        acc |= t[nfa_first(T, G, g) + (((uint32_t)(s >> nfa_shift(T, G, g)) ^ x) & m)];
     }
     return acc;
 }
 
 // Threads take strings first .. first + n - 1 from the counter *head and walk them
 // in 16-byte windows; results go to index i of the output arrays.
-template <int B>
-__device__ __forceinline__ void nfa_walk_queue(const uint64_t *tbl, int sigma, uint64_t start_mask,
+template <int T, int G>
+__device__ __forceinline__ void nfa_walk_queue(const typename NfaWord<T>::type *tbl, int sigma, uint64_t start_mask,
                                                uint64_t accept_mask, const uint8_t *d, int64_t total_bytes,
                                                const int64_t *offsets, int64_t first, int64_t n,
                                                unsigned long long *head, uint32_t *err, uint64_t *final_mask,
@@ -87,9 +105,10 @@ __device__ __forceinline__ void nfa_walk_queue(const uint64_t *tbl, int sigma, u
             atomicOr(err, 1u);
             continue;
         }
-        uint64_t s = start_mask;
+        using W = typename NfaWord<T>::type;
+        W s = (W)start_mask;
         int64_t p = a;
-        while (p < b && (((uintptr_t)(d + p)) & 15u)) s = nfa_step<B>(tbl, s, __ldg(d + p++), sigma);
+        while (p < b && (((uintptr_t)(d + p)) & 15u)) s = nfa_step<T, G>(tbl, s, __ldg(d + p++), sigma);
         if (b - p >= 16) {
             uint4 v = ld_stream16(d + p);
             while (true) {
@@ -98,31 +117,39 @@ __device__ __forceinline__ void nfa_walk_queue(const uint64_t *tbl, int sigma, u
                 if (more) nv = ld_stream16(d + p + 16);
                 const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int k2 = 0; k2 < 16; ++k2) s = nfa_step<B>(tbl, s, (w[k2 >> 2] >> (8 * (k2 & 3))) & 0xffu, sigma);
+                for (int k2 = 0; k2 < 16; ++k2) s = nfa_step<T, G>(tbl, s, (w[k2 >> 2] >> (8 * (k2 & 3))) & 0xffu, sigma);
                 p += 16;
                 if (!more) break;
                 v = nv;
             }
         }
-        while (p < b) s = nfa_step<B>(tbl, s, __ldg(d + p++), sigma);
-        const bool ok = (s & accept_mask) != 0;
+        while (p < b) s = nfa_step<T, G>(tbl, s, __ldg(d + p++), sigma);
+        const bool ok = (s & (W)accept_mask) != 0;
         if (final_mask) final_mask[i] = s;
         if (accept) accept[i] = ok ? 1 : 0;
         if (accept_i32) accept_i32[i] = ok ? 1 : 0;
     }
 }
 
-template <int B, bool SMEM>
+// Copies an automaton's tables into shared memory (16 bytes at a time; the device tables are
+// padded to that).
+extern __shared__ __align__(16) uint8_t s_nfa_tbl[];
+template <int T, int G>
+__device__ __forceinline__ const typename NfaWord<T>::type *nfa_tables_in(const void *tables, int sigma) {
+    using W = typename NfaWord<T>::type;
+    const int n16 = (int)(((size_t)(sigma + 1) * nfa_table_entries(T, G) * sizeof(W) + 15) / 16);
+    const uint4 *src = static_cast<const uint4 *>(tables);
+    uint4 *dst = reinterpret_cast<uint4 *>(s_nfa_tbl);
+    for (int i = threadIdx.x; i < n16; i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+    return reinterpret_cast<const W *>(s_nfa_tbl);
+}
+
+template <int T, int G, bool SMEM>
 __global__ void __launch_bounds__(kNfaThreads, 1) nfa_bitpar_kernel(NfaParams P) {
-    extern __shared__ __align__(16) uint64_t s_tbl[];
-    const uint64_t *tbl = P.tables;
-    if (SMEM) {
-        const int words = (P.sigma + 1) * nfa_table_entries(B);
-        for (int i = threadIdx.x; i < words; i += blockDim.x) s_tbl[i] = P.tables[i];
-        __syncthreads();
-        tbl = s_tbl;
-    }
-    nfa_walk_queue<B>(tbl, P.sigma, P.start_mask, P.accept_mask, P.data, P.total_bytes, P.offsets, 0, P.n,
+    const typename NfaWord<T>::type *tbl = static_cast<const typename NfaWord<T>::type *>(P.tables);
+    if constexpr (SMEM) tbl = nfa_tables_in<T, G>(P.tables, P.sigma);
+    nfa_walk_queue<T, G>(tbl, P.sigma, P.start_mask, P.accept_mask, P.data, P.total_bytes, P.offsets, 0, P.n,
                       P.head, P.err, P.final_mask, P.accept, P.accept_i32);
 }
 
@@ -141,39 +168,53 @@ struct NfaMultiParams {
     unsigned long long *heads;   // one counter a group
     uint32_t *err;
     int n_groups;
-    const uint64_t *tables[kNfaMultiMax];
+    const void *tables[kNfaMultiMax];
     uint64_t start_mask[kNfaMultiMax], accept_mask[kNfaMultiMax];
     int64_t first[kNfaMultiMax], count[kNfaMultiMax];
     int32_t cta_first[kNfaMultiMax + 1];
     int32_t sigma[kNfaMultiMax];
 };
 
-template <int B, bool SMEM>
+template <int T, int G, bool SMEM>
 __global__ void __launch_bounds__(kNfaThreads, 1) nfa_bitpar_multi_kernel(const __grid_constant__ NfaMultiParams P) {
-    extern __shared__ __align__(16) uint64_t s_tbl[];
     int g = 0;
     while (g + 1 < P.n_groups && (int)blockIdx.x >= P.cta_first[g + 1]) ++g;
     const int sigma = P.sigma[g];
-    const uint64_t *tbl = P.tables[g];
-    if (SMEM) {
-        const int words = (sigma + 1) * nfa_table_entries(B);
-        for (int i = threadIdx.x; i < words; i += blockDim.x) s_tbl[i] = tbl[i];
-        __syncthreads();
-        tbl = s_tbl;
-    }
-    nfa_walk_queue<B>(tbl, sigma, P.start_mask[g], P.accept_mask[g], P.data, P.total_bytes, P.offsets,
+    const typename NfaWord<T>::type *tbl = static_cast<const typename NfaWord<T>::type *>(P.tables[g]);
+    if constexpr (SMEM) tbl = nfa_tables_in<T, G>(P.tables[g], sigma);
+    nfa_walk_queue<T, G>(tbl, sigma, P.start_mask[g], P.accept_mask[g], P.data, P.total_bytes, P.offsets,
                       P.first[g], P.count[g], P.heads + g, P.err, P.final_mask, P.accept,
                       P.accept_i32);
+}
+
+// The table layouts, fewest lookups a byte first for each T.
+struct NfaLayout {
+    int T, G;
+    bool smem;
+    void (*run)(NfaParams);
+    void (*run_multi)(NfaMultiParams);
+};
+#define TREX_NFA_LAYOUT(T, G, SMEM) \
+    NfaLayout{T, G, SMEM, nfa_bitpar_kernel<T, G, SMEM>, nfa_bitpar_multi_kernel<T, G, SMEM>}
+static const NfaLayout kNfaLayouts[] = {
+    TREX_NFA_LAYOUT(16, 2, true),  TREX_NFA_LAYOUT(32, 4, true),  TREX_NFA_LAYOUT(32, 5, true),
+    TREX_NFA_LAYOUT(32, 6, true),  TREX_NFA_LAYOUT(32, 7, true),
+    TREX_NFA_LAYOUT(64, 8, true),  TREX_NFA_LAYOUT(64, 9, true),  TREX_NFA_LAYOUT(64, 10, true),
+    TREX_NFA_LAYOUT(64, 11, true), TREX_NFA_LAYOUT(64, 12, true), TREX_NFA_LAYOUT(64, 13, true),
+    TREX_NFA_LAYOUT(64, 16, true), TREX_NFA_LAYOUT(64, 8, false)};
+#undef TREX_NFA_LAYOUT
+static size_t nfa_table_bytes(const NfaLayout &L, int sigma) {
+    return ((size_t)(sigma + 1) * nfa_table_entries(L.T, L.G) * (L.T > 32 ? 8 : 4) + 15) & ~size_t(15);
 }
 
 }  // namespace trex
 
 struct trex_nfa {
-    int n_states = 0, sigma = 0, B = 6;
-    bool smem = true;
+    int n_states = 0, sigma = 0;
+    const trex::NfaLayout *lay = nullptr;   // table layout and its kernels
     uint64_t start_mask = 0, accept_mask = 0;
-    uint64_t *d_tables = nullptr;
-    size_t table_words = 0;
+    uint8_t *d_tables = nullptr;
+    size_t table_bytes = 0;   // a multiple of 16
     void *d_misc = nullptr;   // head counter + error word
     int n_sms = 0;
     std::vector<uint64_t> cols;   // host copy: sigma x 64 destination masks
@@ -182,39 +223,35 @@ struct trex_nfa {
 
 namespace trex {
 
-static void nfa_choose_layout(int sigma, int *B, bool *smem) {
-    // the widest groups (fewest lookups a byte) whose tables fit in shared memory
-    for (int b : {8, 7, 6, 5, 4}) {
-        if ((size_t)(sigma + 1) * nfa_table_entries(b) * 8 <= kNfaSmemBudget) {
-            *B = b;
-            *smem = true;
-            return;
-        }
-    }
-    *B = 8;
-    *smem = false;
+// The first layout that holds the states and whose tables fit in shared memory (the last one
+// stays in global memory).
+static const NfaLayout *nfa_choose_layout(int n_states, int sigma) {
+    const NfaLayout *l = kNfaLayouts;
+    while (l->T < n_states || (l->smem && nfa_table_bytes(*l, sigma) > kNfaSmemBudget)) ++l;
+    return l;
 }
 
-static std::vector<uint64_t> nfa_build_tables(const std::vector<uint64_t> &cols, int sigma, int B,
-                                              int unknown_rejects) {
-    const int G = nfa_groups(B), E = nfa_table_entries(B);
-    std::vector<uint64_t> t((size_t)(sigma + 1) * E, 0);
+// The tables of a layout, in its entry type.
+template <int T>
+static void nfa_build_tables(const std::vector<uint64_t> &cols, int sigma, int G, int unknown_rejects, uint8_t *out) {
+    using W = typename NfaWord<T>::type;
+    const int E = nfa_table_entries(T, G);
+    W *t = reinterpret_cast<W *>(out);
     for (int c = 0; c <= sigma; ++c) {
-        uint64_t *tc = t.data() + (size_t)c * E;
         for (int g = 0; g < G; ++g) {
-            for (int v = 0; v < (1 << B); ++v) {
+            const int width = nfa_width(T, G, g), first = nfa_first(T, G, g), src0 = nfa_shift(T, G, g);
+            const int x = (int)(nfa_swizzle<T>((uint32_t)c) & ((1u << width) - 1u));
+            for (int v = 0; v < (1 << width); ++v) {
                 uint64_t acc = 0;
-                for (int bit = 0; bit < B; ++bit) {
-                    const int src = g * B + bit;
-                    if (!((v >> bit) & 1) || src >= 64) continue;
-                    if (c < sigma) acc |= cols[(size_t)c * 64 + src];
-                    else if (!unknown_rejects) acc |= 1ull << src;   // identity: skip the byte
+                for (int bit = 0; bit < width; ++bit) {
+                    if (!((v >> bit) & 1)) continue;
+                    if (c < sigma) acc |= cols[(size_t)c * 64 + src0 + bit];
+                    else if (!unknown_rejects) acc |= 1ull << (src0 + bit);   // identity: skip the byte
                 }
-                tc[(g << B) + (v ^ (int)(nfa_swizzle((uint32_t)c) & ((1u << B) - 1u)))] = acc;
+                t[(size_t)c * E + first + (v ^ x)] = (W)acc;
             }
         }
     }
-    return t;
 }
 
 int nfa_run(trex_nfa *nfa, const uint8_t *data, const int64_t *offsets, int64_t n,
@@ -241,34 +278,16 @@ int nfa_run(trex_nfa *nfa, const uint8_t *data, const int64_t *offsets, int64_t 
     P.accept_i32 = accept_i32;
     P.head = head;
     P.err = err;
-    const size_t smem = nfa->smem ? nfa->table_words * 8 : 0;
+    const size_t smem = nfa->lay->smem ? nfa->table_bytes : 0;
     // a thread a string: a few strings need one CTA, so that batches of several
     // automata launched on separate streams run side by side
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nfa->n_sms, (n + 31) / 32));
     profile_kernel_begin(stream);
-    switch (nfa->B) {
-        case 8: nfa->smem ? nfa_bitpar_kernel<8, true><<<grid, kNfaThreads, smem, stream>>>(P)
-                          : nfa_bitpar_kernel<8, false><<<grid, kNfaThreads, 0, stream>>>(P); break;
-        case 7: nfa_bitpar_kernel<7, true><<<grid, kNfaThreads, smem, stream>>>(P); break;
-        case 6: nfa_bitpar_kernel<6, true><<<grid, kNfaThreads, smem, stream>>>(P); break;
-        case 5: nfa_bitpar_kernel<5, true><<<grid, kNfaThreads, smem, stream>>>(P); break;
-        default: nfa_bitpar_kernel<4, true><<<grid, kNfaThreads, smem, stream>>>(P); break;
-    }
+    nfa->lay->run<<<grid, kNfaThreads, smem, stream>>>(P);
     TREX_CHECK_LAUNCH();
     profile_kernel_end(stream);
     if (err_out) *err_out = err;
     return TREX_OK;
-}
-
-template <int B, bool SMEM>
-static cudaError_t nfa_multi_launch(const NfaMultiParams &P, int grid, size_t smem, cudaStream_t st) {
-    if (SMEM) {
-        const cudaError_t e = cudaFuncSetAttribute(nfa_bitpar_multi_kernel<B, SMEM>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    nfa_bitpar_multi_kernel<B, SMEM><<<grid, kNfaThreads, SMEM ? smem : 0, st>>>(P);
-    return cudaGetLastError();
 }
 
 int nfa_run_multi(trex_nfa *const *nfas, int n_groups, const int64_t *group_first, const uint8_t *data,
@@ -289,8 +308,7 @@ int nfa_run_multi(trex_nfa *const *nfas, int n_groups, const int64_t *group_firs
     int used_heads = 0;
     for (int g0 = 0; g0 < n_groups; ++g0) {
         if (taken[g0]) continue;
-        const int B = nfas[g0]->B;
-        const bool sm = nfas[g0]->smem;
+        const NfaLayout *lay = nfas[g0]->lay;
         NfaMultiParams P{};
         P.data = data;
         P.total_bytes = total_bytes;
@@ -304,7 +322,7 @@ int nfa_run_multi(trex_nfa *const *nfas, int n_groups, const int64_t *group_firs
         size_t smem = 0;
         for (int g = g0; g < n_groups; ++g) {
             const trex_nfa *h = nfas[g];
-            if (taken[g] || h->B != B || h->smem != sm) continue;
+            if (taken[g] || h->lay != lay) continue;
             taken[g] = true;
             const int64_t cnt = group_first[g + 1] - group_first[g];
             if (cnt == 0) continue;
@@ -317,21 +335,15 @@ int nfa_run_multi(trex_nfa *const *nfas, int n_groups, const int64_t *group_firs
             P.cta_first[k] = ctas;
             // a thread a string, as in a single-automaton run
             ctas += (int)std::max<int64_t>(1, std::min<int64_t>(h->n_sms, (cnt + 31) / 32));
-            smem = std::max(smem, h->table_words * 8);
+            smem = std::max(smem, h->table_bytes);
             ++k;
         }
         if (k == 0) continue;
         P.n_groups = k;
         P.cta_first[k] = ctas;
         used_heads += k;
-        cudaError_t e;
-        switch (B) {
-            case 8: e = sm ? nfa_multi_launch<8, true>(P, ctas, smem, st) : nfa_multi_launch<8, false>(P, ctas, 0, st); break;
-            case 7: e = nfa_multi_launch<7, true>(P, ctas, smem, st); break;
-            case 6: e = nfa_multi_launch<6, true>(P, ctas, smem, st); break;
-            case 5: e = nfa_multi_launch<5, true>(P, ctas, smem, st); break;
-            default: e = nfa_multi_launch<4, true>(P, ctas, smem, st); break;
-        }
+        lay->run_multi<<<ctas, kNfaThreads, lay->smem ? smem : 0, st>>>(P);
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             set_last_error("trex_nfa_run_multi", e);
             return TREX_ERR_CUDA;
@@ -362,9 +374,12 @@ int trex_nfa_create(int n_states, int sigma, const uint64_t *cols, uint64_t star
     nfa->cols.assign((size_t)sigma * 64, 0);
     for (int c = 0; c < sigma; ++c)
         for (int j = 0; j < n_states; ++j) nfa->cols[(size_t)c * 64 + j] = cols[(size_t)c * 64 + j] & keep;
-    nfa_choose_layout(sigma, &nfa->B, &nfa->smem);
-    std::vector<uint64_t> t = nfa_build_tables(nfa->cols, sigma, nfa->B, nfa->unknown_rejects);
-    nfa->table_words = t.size();
+    nfa->lay = nfa_choose_layout(n_states, sigma);
+    nfa->table_bytes = nfa_table_bytes(*nfa->lay, sigma);
+    std::vector<uint8_t> t(nfa->table_bytes);
+    if (nfa->lay->T == 64) nfa_build_tables<64>(nfa->cols, sigma, nfa->lay->G, nfa->unknown_rejects, t.data());
+    else if (nfa->lay->T == 32) nfa_build_tables<32>(nfa->cols, sigma, nfa->lay->G, nfa->unknown_rejects, t.data());
+    else nfa_build_tables<16>(nfa->cols, sigma, nfa->lay->G, nfa->unknown_rejects, t.data());
     nfa->n_sms = sm_count();
     if (nfa->n_sms <= 0) {
         delete nfa;
@@ -372,25 +387,20 @@ int trex_nfa_create(int n_states, int sigma, const uint64_t *cols, uint64_t star
         return TREX_ERR_SHAPE;
     }
     cudaError_t e;
-    if ((e = cudaMalloc(&nfa->d_tables, t.size() * 8)) != cudaSuccess ||
+    if ((e = cudaMalloc(&nfa->d_tables, t.size())) != cudaSuccess ||
         (e = cudaMalloc(&nfa->d_misc, 16)) != cudaSuccess ||
-        (e = cudaMemcpy(nfa->d_tables, t.data(), t.size() * 8, cudaMemcpyHostToDevice)) != cudaSuccess) {
+        (e = cudaMemcpy(nfa->d_tables, t.data(), t.size(), cudaMemcpyHostToDevice)) != cudaSuccess) {
         set_last_error("trex_nfa_create", e);
         cudaFree(nfa->d_tables);
         cudaFree(nfa->d_misc);
         delete nfa;
         return e == cudaErrorMemoryAllocation ? TREX_ERR_OOM : TREX_ERR_CUDA;
     }
-    if (nfa->smem) {
-        const int smem = (int)(t.size() * 8);
-        switch (nfa->B) {
-            case 8: e = cudaFuncSetAttribute(nfa_bitpar_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); break;
-            case 7: e = cudaFuncSetAttribute(nfa_bitpar_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); break;
-            case 6: e = cudaFuncSetAttribute(nfa_bitpar_kernel<6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); break;
-            case 5: e = cudaFuncSetAttribute(nfa_bitpar_kernel<5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); break;
-            default: e = cudaFuncSetAttribute(nfa_bitpar_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); break;
-        }
-        if (e != cudaSuccess) {
+    if (nfa->lay->smem) {
+        // the attribute is per kernel: raised to what any automaton of the layout can need
+        for (const void *f : {(const void *)nfa->lay->run, (const void *)nfa->lay->run_multi}) {
+            if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNfaSmemBudget)) == cudaSuccess)
+                continue;
             set_last_error("trex_nfa_create: cudaFuncSetAttribute", e);
             cudaFree(nfa->d_tables);
             cudaFree(nfa->d_misc);
