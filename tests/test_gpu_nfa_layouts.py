@@ -1,5 +1,5 @@
 """Table layouts of the bit-parallel NFA (group widths, 16-, 32- and 64-state words)
-against the C oracle."""
+and strings cut into units, against the C oracle."""
 
 import numpy as np
 import pytest
@@ -14,9 +14,11 @@ def _run(torch, T, start, acc, data, off, rejects):
     nfa = NFA(T, start, acc, unknown_rejects=rejects)
     d = torch.from_numpy(np.ascontiguousarray(data)).cuda()
     fm, ac = nfa.run(d, torch.from_numpy(off).cuda())
+    fm2, _ = nfa.run(d, torch.from_numpy(off).cuda())   # the handle's units again
     torch.cuda.synchronize()
     err = nfa.error_word()
     nfa.close()
+    assert torch.equal(fm, fm2)
     return fm.cpu().numpy().view(np.uint64), ac.cpu().numpy(), err
 
 
@@ -44,3 +46,50 @@ def test_layouts(cuda, oracle, n, sigma):
     T, start, acc = random_bool_nfa(rng, n, sigma, min(0.5, 2.5 / n))
     data, off = _batch(rng.integers(0, 90, size=300), min(256, sigma + 1), rng)
     _check(cuda, oracle, T, start, acc, data, off, rejects=False)
+
+
+def _shift_nfa(n, sigma):
+    """Every symbol rotates the states: the sets from all states never shrink, no guess holds."""
+    T = np.zeros((sigma, n, n), dtype=np.int8)
+    for c in range(sigma):
+        for j in range(n):
+            T[c, (j + 1 + c) % n, j] = 1
+    start = np.zeros(n, dtype=np.int8)
+    start[0] = 1
+    acc = np.zeros(n, dtype=np.int8)
+    acc[: n // 3 + 1] = 1
+    return T, start, acc
+
+
+def _late_nfa(n, sigma):
+    """Symbol 0 rotates, the others reset to state 0: guesses hold only after a reset, so some
+    units of a string are walked again."""
+    T, start, acc = _shift_nfa(n, sigma)
+    T[1:] = 0
+    T[1:, 0, :] = 1
+    return T, start, acc
+
+
+# around the shortest unit (512 bytes past the first 16-byte boundary), several units, one long
+LENS = {"edges": [0, 1, 15, 16, 511, 512, 513, 526, 527, 528, 529, 1023, 1024, 1025, 1040, 1537, 5000] * 4,
+        "one": [200003], "mixed": [20] * 500 + [30000, 4097, 700] * 3 + [300] * 400}
+
+
+@pytest.mark.parametrize("kind", ["random", "shift", "late", "dies"])
+@pytest.mark.parametrize("shape", sorted(LENS))
+@pytest.mark.parametrize("n", [64, 20])
+def test_strings_cut_into_units(cuda, oracle, kind, shape, n):
+    rng = np.random.default_rng(n + len(kind) + len(shape))
+    sigma = 6
+    data, off = _batch(np.array(LENS[shape], dtype=np.int64), sigma, rng, lead=5)
+    if kind == "random":
+        T, start, acc = random_bool_nfa(rng, n, sigma, 3.0 / n)
+    elif kind == "shift":
+        T, start, acc = _shift_nfa(n, sigma)
+    else:
+        T, start, acc = _late_nfa(n, sigma)
+        data = np.where(rng.random(data.size) < 0.002, data, 0).astype(np.uint8)
+    rejects = kind == "dies"   # a byte outside the alphabet empties the set
+    if rejects:
+        data[rng.integers(0, data.size, size=3)] = sigma + 1
+    _check(cuda, oracle, T, start, acc, data, off, rejects)
