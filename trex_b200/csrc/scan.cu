@@ -11,13 +11,13 @@
 // Design (N <= 16; the per-lane replicated table of dfa_walk.cuh)
 //  * Strings are cut into tiles of tile_len bytes; a warp takes 32
 //    consecutive tiles (a chunk) with one atomic.
-//  * Sync: every lane walks all 16 states of its tile together (16
-//    independent chains) until they coincide, at the same byte offset S for
-//    the whole warp. From there the tile's states no longer depend on its
+//  * Sync: every lane walks all states of its tile together (8 or 16
+//    independent chains, by the table layout) until they coincide, at the
+//    same byte offset S for the whole warp. From there the tile's states no longer depend on its
 //    entry state: its map is constant. A tile that starts a string begins in
 //    the start state and needs no sync.
 //  * Body: each lane walks bytes [tile + S, tile end) with one chain and
-//    writes every state (16-byte stores of packed states).
+//    writes every state (32-byte stores of packed states).
 //  * Entry states: inside the warp, the entry of tile i is the exit of tile
 //    i-1 (a shuffle scan over tile maps handles the general case). Across
 //    warps, chunk c publishes its composed map (AGGREGATE) as soon as its body
@@ -27,8 +27,8 @@
 //    sets the error word and the chunk gives up.
 //  * Head: with the entry state known, each lane walks bytes [tile,
 //    tile + S) again from it and writes those states.
-//  * Tiles whose 16 states never coincide (automata that do not
-//    synchronise) keep all 16 chains over the whole tile, publish the full
+//  * Tiles whose states never coincide (automata that do not
+//    synchronise) keep all chains over the whole tile, publish the full
 //    map and are walked again from their true entry state.
 #include <algorithm>
 #include <cstring>
@@ -37,7 +37,7 @@
 
 namespace trex {
 
-constexpr int kScanThreads = 1024;
+constexpr int kScanThreads = 512;
 constexpr int kSyncCap = 512;                 // bytes walked with 16 chains before giving up
 
 enum : uint32_t { kStAgg = 1u, kStPrefix = 2u };
@@ -72,65 +72,69 @@ static ScanScratch scan_layout(int64_t n_strings, int64_t total_bytes, int32_t t
     return L;
 }
 
-// tile_base[i] = number of tiles of strings 0..i-1 (single block, sequential
-// per thread chunk then a block scan; fine for the few long strings this path
-// is for, and correct for any count). The chunk buffers hold max_tiles tiles,
-// enough for well-formed offsets; overlapping offsets that need more set the
-// capacity bit and leave zero tiles, so the scan kernel touches nothing.
-// Sums saturate at max_tiles + 1 so that they cannot wrap.
-__global__ void scan_tile_base_kernel(const int64_t *offsets, int64_t n, int64_t total_bytes,
-                                      int32_t tile, int64_t max_tiles, int64_t *tile_base,
-                                      uint32_t *err) {
-    __shared__ int64_t part[1024];
-    __shared__ bool over;
-    const int64_t per = (n + blockDim.x - 1) / blockDim.x;
-    const int64_t lo = threadIdx.x * per, hi = min(n, lo + per);
+// One block: tile_base[i] = number of tiles of strings 0..i-1 (each thread its share of the strings
+// in order, a block scan between the shares), the results of empty strings (no tile: the start
+// state), and the cleared chunk status, chunk counter and error word. The chunk buffers hold
+// max_tiles tiles, enough for well-formed offsets; overlapping offsets that need more set the
+// capacity bit and leave zero tiles, so the scan kernel touches nothing. Sums saturate at
+// max_tiles + 1 so that they cannot wrap.
+constexpr int kScanPlanThreads = 1024;
+__global__ void __launch_bounds__(kScanPlanThreads)
+scan_plan_kernel(const int64_t *offsets, int64_t n, int64_t total_bytes, int32_t tile, int64_t max_tiles,
+                 int64_t chunks, int64_t *tile_base, uint32_t *chunk_status, unsigned long long *head, uint32_t *err,
+                 int start, const uint8_t *accept, uint8_t *final_state, uint8_t *acc) {
+    __shared__ int64_t part[kScanPlanThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (int64_t i = threadIdx.x; i < chunks; i += kScanPlanThreads) chunk_status[i] = 0u;
+    if (threadIdx.x == 0) {
+        *head = 0ull;
+        *err = 0u;
+    }
+    __syncthreads();
+    const int64_t per = (n + kScanPlanThreads - 1) / kScanPlanThreads;
+    const int64_t lo = min(n, threadIdx.x * per), hi = min(n, lo + per);
+    // tiles of string i; -1 when it is malformed
+    auto tiles_of = [&](int64_t i) -> int64_t {
+        const int64_t a = offsets[i], b = offsets[i + 1];
+        return a < 0 || b < a || b > total_bytes ? -1 : (b - a + tile - 1) / tile;
+    };
     int64_t sum = 0;
     for (int64_t i = lo; i < hi; ++i) {
-        const int64_t a = offsets[i], b = offsets[i + 1];
-        if (a < 0 || b < a || b > total_bytes) {
+        const int64_t k = tiles_of(i);
+        if (k < 0) {
             atomicOr(err, kScanErrOffsets);
             continue;
         }
-        sum = min(sum + (b - a + tile - 1) / tile, max_tiles + 1);
-    }
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int t = 0; t < (int)blockDim.x; ++t) {
-            const int64_t v = part[t];
-            part[t] = run;
-            run = min(run + v, max_tiles + 1);
-        }
-        over = run > max_tiles;
-        if (over) atomicOr(err, kScanErrCapacity);
-    }
-    __syncthreads();
-    if (over) {
-        for (int64_t i = lo; i < hi; ++i) tile_base[i] = 0;
-        if (threadIdx.x == 0) tile_base[n] = 0;
-        return;
-    }
-    int64_t run = part[threadIdx.x];
-    for (int64_t i = lo; i < hi; ++i) {
-        tile_base[i] = run;
-        const int64_t a = offsets[i], b = offsets[i + 1];
-        if (!(a < 0 || b < a || b > total_bytes)) run += (b - a + tile - 1) / tile;
-    }
-    if (hi == n && lo < n) tile_base[n] = run;
-    if (n == 0 && threadIdx.x == 0) tile_base[0] = 0;
-}
-
-// Empty strings have no tile: their final state is the start state.
-__global__ void scan_empty_kernel(const int64_t *offsets, int64_t n, int start,
-                                  const uint8_t *accept, uint8_t *final_state, uint8_t *acc) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
+        sum = min(sum + k, max_tiles + 1);
         if (offsets[i + 1] == offsets[i]) {
             if (final_state) final_state[i] = (uint8_t)start;
             if (acc) acc[i] = accept[start];
         }
+    }
+    int64_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl = min(incl + v, max_tiles + 1);
+    }
+    if (lane == 31u) part[warp] = incl;
+    __syncthreads();
+    int64_t run = incl - sum, all = 0;   // (incl >= sum also where it saturated)
+    for (uint32_t w = 0; w < kScanPlanThreads / 32; ++w) {
+        if (w == warp) run = min(all + run, max_tiles + 1);
+        all = min(all + part[w], max_tiles + 1);
+    }
+    if (all > max_tiles) {
+        if (threadIdx.x == 0) atomicOr(err, kScanErrCapacity);
+        for (int64_t i = lo; i < hi; ++i) tile_base[i] = 0;
+        if (threadIdx.x == 0) tile_base[n] = 0;
+        return;
+    }
+    for (int64_t i = lo; i < hi; ++i) {
+        tile_base[i] = run;
+        run += max((int64_t)0, tiles_of(i));
+    }
+    if (threadIdx.x == 0) tile_base[n] = all;
 }
 
 // ---- nibble maps (16 states x 4 bits) ----------------------------------------------
@@ -303,28 +307,52 @@ __device__ void scan_chunk(const ScanParams &P, const W &w, int64_t chunk, int64
     const bool have = t < n_tiles;
     TileInfo ti{0, 0, 0, true, false};
     if (have) ti = locate_tile(P, t);
-    // ---- sync: 16 chains until they coincide (same S for the whole warp)
-    uint32_t ch[16];
+    // ---- sync: all states' chains until they coincide (same S for the whole warp); 16 bytes a
+    // step from aligned words (a byte load of 32 tiles touches 32 lines, as a word load does)
+    constexpr int NC = W::kChains;
+    uint32_t ch[NC];
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
+    for (int j = 0; j < NC; ++j)
         ch[j] = w.enc(ti.first ? (uint32_t)P.start : (j < P.n_states ? (uint32_t)j : 0u));
     int64_t S = 0;
     const int64_t len = have ? ti.b1 - ti.b0 : 0;
     bool conv = true;
 #pragma unroll
-    for (int j = 1; j < 16; ++j) conv &= (ch[j] == ch[0]);
+    for (int j = 1; j < NC; ++j) conv &= (ch[j] == ch[0]);
     while (!__all_sync(FULL, conv || S >= len) && S < kSyncCap) {
-        for (int k = 0; k < 16; ++k) {
-            if (S + k < len) {
-                const uint32_t c = __ldg(P.data + ti.b0 + S + k);
+        const int left = (int)min((int64_t)16, max((int64_t)0, len - S));
+        const uint8_t *const p = P.data + ti.b0 + S;
+        uint32_t x[4] = {0u, 0u, 0u, 0u};
+        const uint32_t *const pw = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
+        if (left > 0 && reinterpret_cast<const uint8_t *>(pw) >= P.data &&
+            reinterpret_cast<const uint8_t *>(pw + 5) <= P.data + P.total_bytes) {
+            const uint32_t sh = ((uint32_t)(uintptr_t)p & 3u) * 8u;
+            uint32_t lo = __ldg(pw);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) ch[j] = w.template step<0>(ch[j], c);
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t hi = __ldg(pw + k + 1);
+                x[k] = __funnelshift_r(lo, hi, sh);
+                lo = hi;
+            }
+        } else {
+            for (int k = 0; k < left; ++k) {   // (constant indices: x stays in registers)
+                const uint32_t c = (uint32_t)__ldg(p + k) << (8 * (k & 3));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[i] |= (k >> 2) == i ? c : 0u;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (k < left) {
+                const uint32_t c = (x[k >> 2] >> (8 * (k & 3))) & 0xffu;
+#pragma unroll
+                for (int j = 0; j < NC; ++j) ch[j] = w.template step<0>(ch[j], c);
             }
         }
         S += 16;
         conv = true;
 #pragma unroll
-        for (int j = 1; j < 16; ++j) conv &= (ch[j] == ch[0]);
+        for (int j = 1; j < NC; ++j) conv &= (ch[j] == ch[0]);
     }
     if (S > len) S = len;
     // ---- body (converged) or full map (not converged)
@@ -335,15 +363,15 @@ __device__ void scan_chunk(const ScanParams &P, const W &w, int64_t chunk, int64
             e = walk_write(w, P, ti.b0 + S, ti.b1, e);
             map = map_const(W::dec(e));
         } else {
-            // does not synchronise: carry all 16 chains over the tile
+            // does not synchronise: carry all chains over the tile
             for (int64_t p = ti.b0 + S; p < ti.b1; ++p) {
                 const uint32_t c = __ldg(P.data + p);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) ch[j] = w.template step<0>(ch[j], c);
+                for (int j = 0; j < NC; ++j) ch[j] = w.template step<0>(ch[j], c);
             }
-            map = 0;
+            map = 0;   // (states past NC do not occur)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) map |= (uint64_t)W::dec(ch[j]) << (4 * j);
+            for (int j = 0; j < NC; ++j) map |= (uint64_t)W::dec(ch[j]) << (4 * j);
             if (ti.first) map = map_const(map_at(map, (uint32_t)P.start));
         }
     }
@@ -466,16 +494,12 @@ int trex_dfa_scan_run(trex_dfa_set *set, int dfa_index, const uint8_t *data,
     uint8_t *sc = static_cast<uint8_t *>(scratch);
     const int64_t max_tiles = n_strings + total_bytes / tile_len + 1;
     const int64_t chunks = max_tiles / 32 + 2;
-    TREX_CUDA(cudaMemsetAsync(sc + L.chunk_status, 0, (size_t)chunks * 4, stream));
-    TREX_CUDA(cudaMemsetAsync(sc + L.head, 0, 8, stream));
-    TREX_CUDA(cudaMemsetAsync(sc + L.err, 0, 4, stream));
     int64_t *tile_base = reinterpret_cast<int64_t *>(sc + L.tile_base);
     uint32_t *err = reinterpret_cast<uint32_t *>(sc + L.err);
-    scan_tile_base_kernel<<<1, 1024, 0, stream>>>(offsets, n_strings, total_bytes, tile_len,
-                                                  max_tiles, tile_base, err);
-    TREX_CHECK_LAUNCH();
-    scan_empty_kernel<<<(int)std::min<int64_t>((n_strings + 255) / 256, 4096), 256, 0, stream>>>(
-        offsets, n_strings, start, acc, final_state, accept);
+    scan_plan_kernel<<<1, kScanPlanThreads, 0, stream>>>(
+        offsets, n_strings, total_bytes, tile_len, max_tiles, chunks, tile_base,
+        reinterpret_cast<uint32_t *>(sc + L.chunk_status), reinterpret_cast<unsigned long long *>(sc + L.head), err,
+        start, acc, final_state, accept);
     TREX_CHECK_LAUNCH();
     ScanParams P;
     P.data = data;
