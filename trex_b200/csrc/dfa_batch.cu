@@ -1784,6 +1784,8 @@ __global__ void __launch_bounds__(kComposeThreads) compose_rewalk_kernel(RaggedP
 
 }  // namespace trex
 
+#include "dfa_small.cuh"
+
 struct trex_dfa_set {
     int n_dfas = 0;
     int max_states = 0;
@@ -1834,6 +1836,7 @@ static int dfa_set_run_ex(trex_dfa_set *set, const uint8_t *data, const int64_t 
     const int64_t multi_n = multi ? n_strings : 0;
     const int64_t n = multi ? n_strings * set->n_dfas : n_strings;   // strings walked
     if (n >= (int64_t)0x7fffffff) return TREX_ERR_CAPACITY;
+    const int32_t seg_len_in = seg_len;
     seg_len = effective_seg_len(seg_len);
     if (n == 0) return TREX_OK;
     // bytes walked: every byte once per automaton in a multi-pattern run
@@ -1873,6 +1876,63 @@ static int dfa_set_run_ex(trex_dfa_set *set, const uint8_t *data, const int64_t 
     uint32_t *cta_splits = reinterpret_cast<uint32_t *>(sc + L.cta_splits);
     const uint32_t base_mis = (uint32_t)((uintptr_t)data & 31u);
 
+    RaggedParams P;
+    P.data = data;
+    P.total_bytes = total_bytes;
+    P.offsets = offsets;
+    P.tmaps = set->d_tmaps;
+    P.accepts = set->d_accepts;
+    P.desc = set->d_desc;
+    P.n_dfas = set->n_dfas;
+    P.seg_len = seg_len;
+    P.items = items;
+    P.q_base = q_base;
+    P.q_count = q_count;
+    P.q_head = q_head;
+    P.q_serve = reinterpret_cast<uint32_t *>(sc + L.q_serve);
+    P.q_bytes = q_bytes;
+    P.err = err;
+    P.maps = maps;
+    P.split_list = split_list;
+    P.fix_list = reinterpret_cast<uint2 *>(sc + L.fix_list);
+    P.fix_cap = (uint32_t)std::min<int64_t>(L.fix_cap, 0xffffffffLL);
+    P.fix_tm_bytes = set->tmap_bytes <= kFixSmemBytes ? (uint32_t)set->tmap_bytes : 0u;
+    P.n_fix = reinterpret_cast<uint32_t *>(sc + L.n_fix);
+    P.rw_list = reinterpret_cast<uint32_t *>(sc + L.rw_list);
+    P.n_rw = reinterpret_cast<uint32_t *>(sc + L.n_rw);
+    P.dfa_id = dfa_id;
+    P.n = n;
+    P.max_items = L.max_items;
+    P.base_mis = base_mis;
+    P.multi_n = multi_n;
+    P.final_state = final_state;
+    P.accept = accept;
+    P.accept_i32 = accept_i32;
+    // Small batches at the default item length: one launch (an explicit item length asks for the
+    // planned path). Measured, one launch against planned, us a call: 16 states, strings of 1024
+    // bytes, 16 KiB / 1 / 4 / 8 / 16 MiB: 14 / 15 / 19 / 27 / 37 against 86 / 78 / 101 / 116 / 117;
+    // log-normal strings (median 512): 15 / 33 / 44 / 62 / 83 against 125 / 126 / 147 / 162 / 188;
+    // 16 automata, strings of 64 bytes, 4 / 8 / 16 MiB: 33 / 58 / 108 against 69 / 74 / 84, so
+    // the limits lie at 8 MiB and as many strings as 64-byte ones make.
+    if (seg_len_in <= 0 && n <= kSmallStrings && walked <= kSmallBytes) {
+        const bool in_smem = set->tmap_bytes <= kSmallMapBytes;
+        P.fix_tm_bytes = in_smem ? (uint32_t)set->tmap_bytes : 0u;
+        const int grid = (int)std::min<int64_t>(
+            set->n_sms, std::max<int64_t>((n + 7) / 8, walked / (32 * kSmallPieceWindows)));
+        // report counters and records of long strings, in the room for work items (32 bytes for
+        // every 2048 bytes of the batch; at most 8 for every kSmallLongBytes here)
+        uint32_t *cnt = reinterpret_cast<uint32_t *>(items);
+        const int64_t max_long = walked / kSmallLongBytes + 1;
+        if (max_long > 1) TREX_CUDA(cudaMemsetAsync(cnt, 0, (size_t)max_long * 4, stream));
+        profile_kernel_begin(stream);
+        if (in_smem) dfa_small_kernel<true><<<grid, kSmallThreads, set->tmap_bytes, stream>>>(P, cnt, cnt + max_long);
+        else dfa_small_kernel<false><<<grid, kSmallThreads, 0, stream>>>(P, cnt, cnt + max_long);
+        TREX_CHECK_LAUNCH();
+        profile_kernel_end(stream);
+        if (err_word_out) *err_word_out = err;
+        return TREX_OK;
+    }
+
     // Queue bases, counts and heads, byte counts, the error word and the item
     // count are contiguous at the front of the scratch buffer.
     TREX_CUDA(cudaMemsetAsync(sc, 0, L.items, stream));
@@ -1898,39 +1958,7 @@ static int dfa_set_run_ex(trex_dfa_set *set, const uint8_t *data, const int64_t 
         cta_bins, bin_base, bin_end, cta_maps, cta_splits, items, L.max_items, split_list, err);
     TREX_CHECK_LAUNCH();
 
-    RaggedParams P;
-    P.data = data;
-    P.total_bytes = total_bytes;
-    P.offsets = offsets;
-    P.tmaps = set->d_tmaps;
-    P.accepts = set->d_accepts;
-    P.desc = set->d_desc;
-    P.n_dfas = set->n_dfas;
-    P.seg_len = seg_len;
-    P.items = items;
-    P.q_base = q_base;
-    P.q_count = q_count;
-    P.q_head = q_head;
-    P.q_serve = reinterpret_cast<uint32_t *>(sc + L.q_serve);
-    P.q_bytes = q_bytes;
-    P.err = err;
-    P.maps = maps;
-    P.split_list = split_list;
     P.n_split = cta_splits + plan_grid;
-    P.fix_list = reinterpret_cast<uint2 *>(sc + L.fix_list);
-    P.fix_cap = (uint32_t)std::min<int64_t>(L.fix_cap, 0xffffffffLL);
-    P.fix_tm_bytes = set->tmap_bytes <= kFixSmemBytes ? (uint32_t)set->tmap_bytes : 0u;
-    P.n_fix = reinterpret_cast<uint32_t *>(sc + L.n_fix);
-    P.rw_list = reinterpret_cast<uint32_t *>(sc + L.rw_list);
-    P.n_rw = reinterpret_cast<uint32_t *>(sc + L.n_rw);
-    P.dfa_id = dfa_id;
-    P.n = n;
-    P.max_items = L.max_items;
-    P.base_mis = base_mis;
-    P.multi_n = multi_n;
-    P.final_state = final_state;
-    P.accept = accept;
-    P.accept_i32 = accept_i32;
     profile_kernel_begin(stream);
     // one CTA per 64 KiB of input (and at least one per automaton the batch may
     // use), at most one per SM: a small batch (a serving batch) then needs a few
@@ -2045,6 +2073,9 @@ int trex_dfa_set_create(int n_dfas, const int32_t *n_states, const int32_t *star
         return fail(e, "cudaFuncSetAttribute");
     if ((e = cudaFuncSetAttribute(trex::compose_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)trex::kFixSmemBytes)) != cudaSuccess)
+        return fail(e, "cudaFuncSetAttribute");
+    if ((e = cudaFuncSetAttribute(trex::dfa_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)trex::kSmallMapBytes)) != cudaSuccess)
         return fail(e, "cudaFuncSetAttribute");
     *out = set;
     return TREX_OK;
