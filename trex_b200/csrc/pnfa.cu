@@ -1780,6 +1780,8 @@ pnfa_chain_kernel(PnPlainParams P, const uint16_t *T16, int resc) {
 
 }  // namespace trex
 
+#include "pnfa_fp32.cuh"
+
 // ---- handle -----------------------------------------------------------------------------------
 struct trex_pnfa {
     int n_states = 0, sigma = 0, npairs = 0, n_sms = 0;
@@ -1832,6 +1834,31 @@ static void pn_free(trex_pnfa *h) {
 
 static int64_t pn_sms(const trex_pnfa *h) {
     return h->sm_limit > 0 ? std::min(h->sm_limit, h->n_sms) : h->n_sms;
+}
+
+// Tables, rings, slots and shared-memory layout of a run of pnfa_fp32_kernel: one CTA an SM, the
+// strings spread over all SMs, as many slots a CTA as it has strings or fit beside the tables.
+static SyParams sy_params(const trex_pnfa *h, int64_t n) {
+    SyParams Q{};
+    Q.T32 = h->d_T32;
+    Q.start_img = reinterpret_cast<const uint4 *>(h->d_start32);
+    Q.acc = h->d_acc;
+    Q.ll_empty = h->ll_empty;
+    Q.wait_cycles = mbar_wait_cycles();
+    Q.sigma = h->sigma;
+    Q.rep = std::max(1, kSyWarps / h->sigma);
+    Q.n_rings = Q.sigma * Q.rep;
+    Q.grid = (int)std::max<int64_t>(1, std::min<int64_t>(n, pn_sms(h)));
+    Q.slots = (int)std::min<int64_t>((n + Q.grid - 1) / Q.grid, kSyMaxSlots);
+    for (;; --Q.slots) {
+        Q.rep_shift = 5;
+        while ((1 << Q.rep_shift) < Q.slots) ++Q.rep_shift;
+        Q.ring_cap = 1 << Q.rep_shift;
+        Q.recs_off = pn_align16(kSyRings + (uint32_t)(Q.n_rings + 1) * (uint32_t)Q.ring_cap * 2u);
+        Q.rows_off = Q.recs_off + (uint32_t)Q.slots * kSyRecBytes;
+        Q.tbl_off = Q.rows_off + (uint32_t)Q.slots * kSyRowBytes;
+        if (Q.tbl_off + (uint32_t)Q.sigma * kSyTblBytes <= kPnSmemCap) return Q;
+    }
 }
 
 static int pn_choose(const trex_pnfa *h, int64_t n, int *grid, int *p_sub) {
@@ -1982,6 +2009,8 @@ int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start
     if (e == cudaSuccess) e = cudaMalloc(&h->d_misc, 16);
     if (e == cudaSuccess) e = cudaMemset(h->d_misc, 0, 16);
     if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(pnfa_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPnSmemCap);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(pnfa_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kPnSmemCap);
     if (e == cudaSuccess)
@@ -2058,6 +2087,25 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
             else
                 pnfa_chain_kernel<false><<<grid, kChainThreads * kChainGroups, smem, st>>>(Q, h->d_T16[0],
                                                                                            h->chain_resc[0]);
+            profile_kernel_end(st);
+            TREX_CHECK_LAUNCH();
+            return TREX_OK;
+        }
+        // alphabets whose tables fit on an SM: strings in rings by symbol (8192 strings x 512, 20
+        // symbols: 1.73 ms against 16.7); larger ones read every table through L1 and L2
+        if (h->sigma <= kSyWarps) {
+            SyParams S = sy_params(h, n_strings);
+            S.data = data;
+            S.total_bytes = total_bytes;
+            S.offsets = offsets;
+            S.n = n_strings;
+            S.loglik = loglik;
+            S.accept = accept;
+            S.accept_i32 = accept_i32;
+            S.queue = queue;
+            S.err = err;
+            profile_kernel_begin(st);
+            pnfa_fp32_kernel<<<S.grid, 32 * S.n_rings, S.tbl_off + (uint32_t)S.sigma * kSyTblBytes, st>>>(S);
             profile_kernel_end(st);
             TREX_CHECK_LAUNCH();
             return TREX_OK;
