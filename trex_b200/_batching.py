@@ -14,10 +14,10 @@ def pack_strings(strings, offset_dtype=np.int32):
     B = len(strings)
     if B and isinstance(strings[0], (bytes, bytearray, memoryview)):
         blob = b"".join(strings)
-        lens = np.fromiter((len(s) for s in strings), dtype=np.int64, count=B)
+        lens = np.fromiter(map(len, strings), dtype=np.int64, count=B)
     else:
         blob = "".join(strings).encode("latin-1")
-        lens = np.fromiter((len(s) for s in strings), dtype=np.int64, count=B)
+        lens = np.fromiter(map(len, strings), dtype=np.int64, count=B)
     offsets = np.zeros(B + 1, dtype=np.int64)
     np.cumsum(lens, out=offsets[1:])
     if offset_dtype == np.int32 and B and offsets[-1] > np.iinfo(np.int32).max:

@@ -1807,9 +1807,9 @@ struct trex_dfa_set {
     uint8_t *st_data = nullptr;
     int64_t *st_off = nullptr;
     int32_t *st_ids = nullptr;
-    uint8_t *st_out = nullptr;     // final_state[n] | accept[n]
-    int32_t *st_out32 = nullptr;
+    uint8_t *st_out = nullptr;     // error word, accept_i32[n], final_state[n], accept[n]: one copy back
     int64_t st_data_cap = 0, st_n_cap = 0;
+    std::vector<uint8_t> h_out;    // their host copy
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 };
 
@@ -2091,7 +2091,6 @@ void trex_dfa_set_destroy(trex_dfa_set *set) {
     cudaFree(set->st_off);
     cudaFree(set->st_ids);
     cudaFree(set->st_out);
-    cudaFree(set->st_out32);
     for (auto &e : set->ev)
         if (e) cudaEventDestroy(e);
     delete set;
@@ -2120,16 +2119,13 @@ int trex_dfa_batch_host(trex_dfa_set *set, const uint8_t *h_data, const int64_t 
         cudaFree(set->st_off);
         cudaFree(set->st_ids);
         cudaFree(set->st_out);
-        cudaFree(set->st_out32);
         set->st_off = nullptr;
         set->st_ids = nullptr;
         set->st_out = nullptr;
-        set->st_out32 = nullptr;
         set->st_n_cap = 0;
         TREX_CUDA(cudaMalloc(&set->st_off, (n + 1) * 8));
         TREX_CUDA(cudaMalloc(&set->st_ids, n * 4));
-        TREX_CUDA(cudaMalloc(&set->st_out, n * 2));
-        TREX_CUDA(cudaMalloc(&set->st_out32, n * 4));
+        TREX_CUDA(cudaMalloc(&set->st_out, 4 + n * 6));
         set->st_n_cap = n;
     }
     for (auto &e : set->ev)
@@ -2141,24 +2137,44 @@ int trex_dfa_batch_host(trex_dfa_set *set, const uint8_t *h_data, const int64_t 
     TREX_CUDA(cudaMemcpyAsync(set->st_off, h_offsets, (n + 1) * 8, cudaMemcpyHostToDevice, st));
     if (h_dfa_id) TREX_CUDA(cudaMemcpyAsync(set->st_ids, h_dfa_id, n * 4, cudaMemcpyHostToDevice, st));
     TREX_CUDA(cudaEventRecord(set->ev[1], st));
+    // outputs: the error word, then the requested arrays back to back
+    const int64_t i32_at = 4, fs_at = i32_at + (h_accept_i32 ? 4 * n : 0), ac_at = fs_at + (h_final_state ? n : 0),
+                  out_end = ac_at + (h_accept ? n : 0);
     uint32_t *err = nullptr;
-    int rc = trex::dfa_set_run(set, set->st_data, set->st_off, h_dfa_id ? set->st_ids : nullptr, n,
-                               total_bytes, h_final_state ? set->st_out : nullptr,
-                               h_accept ? set->st_out + n : nullptr,
-                               h_accept_i32 ? set->st_out32 : nullptr, nullptr, 0, seg_len, st,
-                               &err);
+    int rc = trex::dfa_set_run(set, set->st_data, set->st_off, h_dfa_id ? set->st_ids : nullptr, n, total_bytes,
+                               h_final_state ? set->st_out + fs_at : nullptr, h_accept ? set->st_out + ac_at : nullptr,
+                               h_accept_i32 ? reinterpret_cast<int32_t *>(set->st_out + i32_at) : nullptr, nullptr, 0,
+                               seg_len, st, &err);
     if (rc) return rc;
     TREX_CUDA(cudaEventRecord(set->ev[2], st));
-    if (h_final_state)
-        TREX_CUDA(cudaMemcpyAsync(h_final_state, set->st_out, n, cudaMemcpyDeviceToHost, st));
-    if (h_accept)
-        TREX_CUDA(cudaMemcpyAsync(h_accept, set->st_out + n, n, cudaMemcpyDeviceToHost, st));
-    if (h_accept_i32)
-        TREX_CUDA(cudaMemcpyAsync(h_accept_i32, set->st_out32, n * 4, cudaMemcpyDeviceToHost, st));
     uint32_t h_err = 0;
-    TREX_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, st));
+    // Each copy to pageable memory is a synchronisation of its own (about 10 us): small batches
+    // come back in one copy and are dealt out here, large ones go straight to the caller's arrays.
+    const bool together = n <= 65536;
+    if (together) {
+        TREX_CUDA(cudaMemcpyAsync(set->st_out, err, 4, cudaMemcpyDeviceToDevice, st));
+        try {
+            set->h_out.resize((size_t)out_end);
+        } catch (const std::bad_alloc &) {
+            return TREX_ERR_OOM;
+        }
+        TREX_CUDA(cudaMemcpyAsync(set->h_out.data(), set->st_out, (size_t)out_end, cudaMemcpyDeviceToHost, st));
+    } else {
+        if (h_final_state)
+            TREX_CUDA(cudaMemcpyAsync(h_final_state, set->st_out + fs_at, n, cudaMemcpyDeviceToHost, st));
+        if (h_accept) TREX_CUDA(cudaMemcpyAsync(h_accept, set->st_out + ac_at, n, cudaMemcpyDeviceToHost, st));
+        if (h_accept_i32)
+            TREX_CUDA(cudaMemcpyAsync(h_accept_i32, set->st_out + i32_at, n * 4, cudaMemcpyDeviceToHost, st));
+        TREX_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, st));
+    }
     TREX_CUDA(cudaEventRecord(set->ev[3], st));
     TREX_CUDA(cudaEventSynchronize(set->ev[3]));
+    if (together) {
+        std::memcpy(&h_err, set->h_out.data(), 4);
+        if (h_accept_i32) std::memcpy(h_accept_i32, set->h_out.data() + i32_at, (size_t)n * 4);
+        if (h_final_state) std::memcpy(h_final_state, set->h_out.data() + fs_at, (size_t)n);
+        if (h_accept) std::memcpy(h_accept, set->h_out.data() + ac_at, (size_t)n);
+    }
     if (kernel_ms) TREX_CUDA(cudaEventElapsedTime(kernel_ms, set->ev[1], set->ev[2]));
     if (total_ms) TREX_CUDA(cudaEventElapsedTime(total_ms, set->ev[0], set->ev[3]));
     if (h_err) {

@@ -86,7 +86,7 @@ class _DfaEngine:
     def run(self, strings):
         data, off = self._pack(strings)
         _, acc, kms, tms = self.set.run_host(data, off)
-        return [bool(a) for a in acc[:len(strings)]], kms, tms
+        return acc[:len(strings)].astype(bool).tolist(), kms, tms
 
     def close(self):
         self.set.close()
