@@ -1,0 +1,37 @@
+"""Planned DFA batches (an explicit item length): the strings' shares of the planning CTAs,
+against the oracle."""
+
+import numpy as np
+import pytest
+
+from trex_b200.workloads import random_dfa
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(torch, oracle, dfas, data, off, ids, seg_len):
+    from trex_b200.engine import DFASet
+    s = DFASet(dfas)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    fs, ac, _ = s.run(up(data), up(off), up(ids), seg_len=seg_len)
+    torch.cuda.synchronize()
+    assert s.last_error_word() == 0
+    s.close()
+    rfs, rac = oracle.dfa_walk([d.tmap for d in dfas], [d.n_states for d in dfas], [d.start for d in dfas],
+                               [d.accept for d in dfas], data, off, ids)
+    assert np.array_equal(fs.cpu().numpy(), rfs)
+    assert np.array_equal(ac.cpu().numpy(), rac)
+
+
+# fewer tiles of 1024 strings than CTAs, as many, a few more, uneven shares
+@pytest.mark.parametrize("n", [1, 1024, 1025, 148 * 1024 - 1, 148 * 1024, 148 * 1024 + 1, 333333])
+def test_shares_of_the_planning_ctas(cuda, oracle, n):
+    rng = np.random.default_rng(n)
+    dfas = [random_dfa(k, np.arange(256), rng) for k in (5, 12, 40)]
+    lens = rng.integers(0, 24, size=n)
+    lens[rng.integers(0, n, size=50)] = 700   # a few of several items
+    off = np.zeros(n + 1, dtype=np.int64)
+    np.cumsum(lens, out=off[1:])
+    data = rng.integers(0, 256, size=int(off[-1]), dtype=np.uint8)
+    ids = rng.integers(0, len(dfas), size=n).astype(np.int32)
+    _check(cuda, oracle, dfas, data, off, ids, 256)
