@@ -35,3 +35,14 @@ def test_shares_of_the_planning_ctas(cuda, oracle, n):
     data = rng.integers(0, 256, size=int(off[-1]), dtype=np.uint8)
     ids = rng.integers(0, len(dfas), size=n).astype(np.int32)
     _check(cuda, oracle, dfas, data, off, ids, 256)
+
+
+# the shared-memory table of each layout: its fewest and most states, and a partial last word
+@pytest.mark.parametrize("n_states", [1, 3, 7, 8, 9, 13, 16, 17, 31, 32, 33, 62, 64, 65])
+def test_tables_of_each_layout(cuda, oracle, n_states):
+    rng = np.random.default_rng(n_states)
+    dfas = [random_dfa(n_states, np.arange(256), rng) for _ in range(2)]
+    off = np.arange(0, 4001, dtype=np.int64) * 300
+    data = rng.integers(0, 256, size=int(off[-1]), dtype=np.uint8)
+    ids = rng.integers(0, 2, size=4000).astype(np.int32)
+    _check(cuda, oracle, dfas, data, off, ids, 256)
