@@ -20,7 +20,7 @@ Workloads (synthetic, seeded; the reference ships no dataset):
       --serve-rates) through trex_b200.serving.Server; reports throughput
       and p50/p99 latency per rate and the plain per-request launch.
   pnfa: probabilistic 64-state NFA over 20 symbols (rows Dirichlet(0.5) x 0.9,
-      ~30% kept), 64K strings x 2048 symbols, tcgen05 kernel with BF16 (or
+      ~30% kept), 64K strings x 2048 symbols, tensor-core kernel with BF16 (or
       --pnfa-mode fp16 / fp32) operands; also reports the log-likelihood error
       against the FP64 oracle.
 
@@ -528,7 +528,7 @@ class NFAWorkload:
 
 
 class PNFAWorkload:
-    """Probabilistic NFA, 64 states, 20 symbols (tcgen05 kernel, or the FP32 kernel)."""
+    """Probabilistic NFA, 64 states, 20 symbols (tensor-core kernel, or the FP32 kernel)."""
 
     kind = "pnfa"
     launches_per_step = 1
@@ -547,13 +547,13 @@ class PNFAWorkload:
         self.L = getattr(args, "nfa_len", None) or 2048
         self.off = np.arange(self.n + 1, dtype=np.int64) * self.L
         # alphabets of at most four symbols run one string a TMEM lane
-        self.kernel = ("pnfa_plain_kernel" if self.mode == "fp32" else
-                       "pnfa_lane_kernel" if self.sigma <= 4 else "pnfa_tc_kernel")
+        self.kernel = ("pnfa_fp32_kernel" if self.mode == "fp32" else
+                       "pnfa_lane_kernel" if self.sigma <= 4 else "pnfa_sym_kernel")
         self.dtype = {"bf16": "bf16", "fp16": "f16", "fp32": "f32"}[self.mode]
         self.workload = (f"probabilistic NFA: 64 states, {self.sigma} symbols (bytes 0..{self.sigma - 1}), rows of T[c] "
                          "Dirichlet(0.5) x 0.9 with ~30% kept, start e0, accept all states; "
                          f"{self.n} strings x {self.L} symbols; {self.mode} operands"
-                         + ("" if self.mode == "fp32" else ", FP32 accumulation (tcgen05)"))
+                         + ("" if self.mode == "fp32" else ", FP32 accumulation (tensor cores)"))
 
     def setup(self, torch, dev, seed):
         from trex_b200.engine import PNFA
@@ -678,10 +678,10 @@ class NFATcWorkload(PNFAWorkload):
         self.n = args.strings or 262144
         self.L = getattr(args, "nfa_len", None) or 4096
         self.off = np.arange(self.n + 1, dtype=np.int64) * self.L
-        self.kernel = "pnfa_lane_kernel" if self.sigma <= 4 else "pnfa_tc_kernel"
+        self.kernel = "pnfa_lane_kernel" if self.sigma <= 4 else "pnfa_sym_kernel"
         self.dtype = "s8" if self.mode == "bool8" else "bf16"
-        ops = ("0/1 int8 operands, int32 sums (tcgen05 kind::i8)" if self.mode == "bool8"
-               else "0/1 BF16 operands, FP32 sums (tcgen05 kind::f16)")
+        ops = ("0/1 int8 operands, int32 sums (tensor cores)" if self.mode == "bool8"
+               else "0/1 BF16 operands, FP32 sums (tensor cores)")
         self.workload = (f"Boolean NFA: random 64-state NFA over {self.sigma} symbols (bytes "
                          f"0..{self.sigma - 1}), edge density 0.05, {self.n} strings x {self.L} symbols; "
                          f"tensor cores, {ops} thresholded every step")
@@ -914,7 +914,7 @@ def serve_measure(args) -> dict:
         "parallelism": "1 GPU, continuous batching (2 lanes x 2 slots, "
                        + ("direct launches)" if args.serve_no_graphs else "CUDA graphs for DFA batches)"),
         "hbm_budget_bytes": 2 << 30,
-        "pnfa_mode": "auto (BF16 tables on CUDA cores below 2048 strings a group, tcgen05 above)",
+        "pnfa_mode": "auto (BF16 tables on CUDA cores below 2048 strings a group, tensor cores above)",
         "value": top["gchar_s"], "unit": "Gchar/s",
         "sustained_req_s": top["offered_req_s"], "p50_ms_at_sustained": top["p50_ms"],
         "p99_ms_at_sustained": top["p99_ms"], "limiter": limiter,

@@ -45,8 +45,8 @@ const char *trex_version(void);
 /* Limits of the bounded device waits (no counterpart in the reference, whose
  * look-back spins without a limit, cuda/monoid_scan.cu:187-193): scan_polls =
  * polls of one look-back step of trex_dfa_scan_run, mbar_cycles = clock cycles
- * of one hand-off wait inside the tensor-core NFA kernel (trex_pnfa_run modes
- * BF16, FP16, BOOL, BOOL8). A wait that runs out sets the timeout bit (4) of
+ * of one hand-off inside the NFA kernels (trex_pnfa_run modes BF16, FP16, BOOL,
+ * BOOL8, FP32). A wait that runs out sets the timeout bit (4) of
  * the run's error word and the kernel returns; the results of that run are
  * then invalid. 0 restores a default (2^24 polls; 4e9 cycles, about 2 s).
  * Process-wide, read at each launch; meant for tests of the give-up paths. */
@@ -311,7 +311,7 @@ enum {
 int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start,
                      const float *accept, trex_pnfa **out);
 void trex_pnfa_destroy(trex_pnfa *pnfa);
-/* mode TREX_PNFA_BF16 / TREX_PNFA_FP16: tensor-core products (tcgen05) with
+/* mode TREX_PNFA_BF16 / TREX_PNFA_FP16: tensor-core products with
  * 16-bit operands and FP32 accumulation, sigma <= 28 (else TREX_ERR_SHAPE);
  * TREX_PNFA_FP32: FP32 on CUDA cores, any sigma. Every step renormalises the
  * state by a power of two kept as an integer exponent.
@@ -323,12 +323,13 @@ void trex_pnfa_destroy(trex_pnfa *pnfa);
  * integers in FP32); accept = some accepting state is active, and loglik is
  * the log of the number of active accepting states. sigma <= 28.
  * TREX_PNFA_BOOL8: the same Boolean NFA with 0/1 int8 operands and int32
- * sums (tcgen05 kind::i8: K = 32 an instruction, so half the MMA
- * instructions of TREX_PNFA_BOOL), thresholded to {0, 1} every step (exact).
+ * sums (K = 32 an MMA instruction, so half the instructions of
+ * TREX_PNFA_BOOL), thresholded to {0, 1} every step (exact).
  * The four tensor-core modes run with sigma <= 4 on a kernel that keeps one
- * string on each TMEM lane (the symbol folded into K: no sorting of strings by
- * symbol; 2-4x the throughput), above it on the kernel that groups strings by
- * symbol pair each step; results are the same within each mode's rounding.
+ * string on each TMEM lane (tcgen05, the symbol folded into K), above it on a
+ * kernel whose warps each keep one symbol's table in registers (mma.sync) and
+ * advance all of a CTA's strings one symbol a step; results are the same within
+ * each mode's rounding.
  * TREX_PNFA_BF16_CC / TREX_PNFA_FP16_CC: CUDA cores with the 16-bit tables in
  * shared memory and an FP32 state, four warps per string: the low-latency form
  * for few (possibly long) strings, sigma <= 28. DEVICE buffers;

@@ -16,57 +16,12 @@
 // l + 32, T[c] rows read through L1; f = the frexp exponent of the step's
 // max |s'|, the rule of the FP64 oracle.
 //
-// Tensor form (tcgen05, BF16 or FP16 operands, FP32 accumulation in TMEM).
-// One persistent CTA per SM holds up to 512 strings ("slots") and advances
-// them all one symbol per step. A tcgen05.mma (M=128, K=16) costs about the
-// same time for any N up to 256 (measured: ~120-165 cycles whether N is 16 or
-// 192), so the kernel is bound by the number of MMA instructions per step:
-// every pair of symbols gets one MMA chain over all of the CTA's strings that
-// carry it (about 40 instructions a step), and chunks pipeline inside a step
-// (the MMA of one symbol pair runs while the epilogue drains the previous
-// one). Orientation: D[dst][string] = T[c][dst][:] . S[:][string]
-// -- the 64 states are the MMA's M rows (TMEM lanes) and the strings its N
-// columns, because strings of one step carry different symbols and only the
-// N side can be regrouped cheaply. Symbols are paired (2p, 2p+1): the A
-// operand of pair p is [T[2p]; T[2p+1]] (M = 128), resident in TMEM for the
-// whole kernel (32 columns a pair: 64 16-bit K values per lane), so the shared
-// memory traffic of an MMA is only its B columns. Each step, the strings of a
-// sub-batch are grouped by pair in the B buffer (even symbol first), and one
-// MMA chain (K = 64 as 4 x K16) per group of <= 64 strings writes a 64-column
-// region of a TMEM ring. Rows 0-63 of the result are valid for the even-symbol
-// strings, rows 64-127 for the odd ones (half the MMA work is discarded: the
-// price of keeping A in TMEM and B small).
-//
-// Warp roles (480 threads):
-//  * warps 0-7, epilogue, two sets of four taking alternate chunks (warp q of a
-//    set reads TMEM lanes 32q..32q+31 with 16x256b loads, four states of four
-//    columns a thread): it scales each string's states by the record's 2^-f,
-//    rounds them to 16 bits, stores them in pairs in the string's row of the
-//    next B buffer and records max|s_t+1| (a butterfly max); on a string's
-//    last symbol it writes the accept-weighted sum instead.
-//  * warp 8, MMA: per chunk waits for a free ring region, issues 4
-//    tcgen05.mma (A from TMEM, B from shared memory, no swizzle) and commits
-//    to the region's mbarrier.
-//  * warps 9-12, planner: per step and sub-batch, sorts the slots of the step
-//    by symbol pair (counting sort with shared atomics), writes the chunk list
-//    and the start vector into the rows of strings that begin; for the
-//    previous step it writes one record per row: the string's row in the next
-//    B buffer and the scale 2^-f, f = the exponent of max|s| * R_c (R_c = max
-//    row sum of |T[c]|, so max|s'| < 1; max|s| left by the epilogue), adding f
-//    to the string's exponent sum; and it turns finished strings' dot
-//    products and exponents into the FP64 log-likelihood.
-//  * warps 13-14, loader: gives each slot its next string from a global
-//    atomic queue and copies the next 16 valid symbols of every slot into a
-//    shared block (strings change slots only at 16-step block boundaries).
-// Hand-offs are mbarriers (one per sub-batch and step parity, so no waiter is
-// ever two phases behind); the planner warps meet at a named barrier and only
-// their leader waits on mbarriers. B buffers (shared memory, K-major, no
-// swizzle): row r, state k at (k/8)*LBO + r*16 + (k%8)*2 with LBO = rows*16 and
-// rows = 1 (mod 8), so the 32 lanes of an epilogue store hit 32 different banks
-// and an MMA may start at any row.
-// Every wait is bounded; one that runs out sets the error word (bit 2) and an
-// abort flag that every role polls; the MMA warp drains its commits and the
-// TMEM is freed before the kernel returns.
+// Tensor forms (BF16, FP16, Boolean): alphabets of up to four symbols keep a string on
+// each TMEM lane and fold the symbol into K (tcgen05, below); larger ones keep a symbol's
+// table in each warp's registers and bring the strings to it (mma.sync, pnfa_sym.cuh). FP32:
+// tables on the SM (pnfa_fp32.cuh), or through L1 for alphabets that do not fit. The
+// low-latency forms with 16-bit tables are at the end.
+// Every wait is bounded; one that runs out sets the error word (bit 2).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -81,144 +36,14 @@
 namespace trex {
 
 constexpr int kPnStates = 64;
-constexpr int kPnBlk = 16;             // steps per symbol block
-constexpr int kPnEpiWarps = 8, kPnMmaWarp = 8, kPnPlanWarp0 = 9, kPnPlanWarps = 4,
-              kPnLoadWarp0 = 13, kPnLoadWarps = 2;
-constexpr int kPnThreads = 32 * (kPnLoadWarp0 + kPnLoadWarps);
-constexpr int kPnPlanThreads = 32 * kPnPlanWarps;
-constexpr int kPnMaxPSub = 512;        // slots per sub-batch
-constexpr int kPnSlotsPerPlanThread = kPnMaxPSub / kPnPlanThreads;
-constexpr int kPnMaxChunks = 32;
-constexpr int kPnRegionCols = 64;
-constexpr int kPnMaxRegions = 6;
-constexpr int kPnMaxSigmaTc = 28;      // 14 pairs: 448 TMEM columns + one ring region
-constexpr int kPnMiscBytes = 2048;
 constexpr uint32_t kPnSmemCap = 232448;
-constexpr int32_t kPnTerminate = -1;
 constexpr uint32_t kPnErrOffsets = 1u, kPnErrTimeout = 4u;
 // The drain of committed MMAs before the TMEM is freed always waits up to the
 // default limit (an MMA still writing TMEM must not outlive the allocation);
 // the hand-off waits use PnParams::wait_cycles.
 constexpr long long kPnDrainCycles = kDefaultMbarCycles;
 
-constexpr uint32_t kRecFinish = 1u << 31;
-// slot flags (planner)
-constexpr uint8_t kSlotActive = 1, kSlotLast = 2, kSlotFresh = 4;
-// header flags (loader)
-constexpr uint8_t kHdrStart = 1, kHdrEnd = 2;
-
-struct PnHdr {
-    int32_t seq;
-    uint8_t count, flags;
-    uint16_t pad;
-};
-struct PnSlot {
-    int32_t seq;          // string in the slot
-    int32_t pend[2];      // string whose last step (of that parity) awaits its log-likelihood
-    int16_t row;          // row at the last planned step
-    uint8_t c, flags, blkcnt, blkflags;
-};
-struct PnChunk {
-    uint16_t row0;
-    uint8_t ncols, split, pair, pad0, pad1, pad2;
-};
-
-struct PnLayout {
-    int p_sub, rows, npairs, nregions, ring_base;
-    uint32_t lbo;
-    uint32_t s_off, sym_off, hdr_off, rec_off, xmax_off, fin_off, fine_off, e_off, chunk_off,
-        slot_off, misc_off, total;
-};
-
 __host__ __device__ inline uint32_t pn_align16(uint32_t x) { return (x + 15u) & ~15u; }
-
-// acols: TMEM columns of a symbol pair's A operand (32 for 16-bit operands: 64 K
-// values of 2 bytes a lane; 16 for int8 operands: 4 K values a 32-bit column).
-static PnLayout pn_layout(int p_sub, int sigma, int acols = 32) {
-    PnLayout L{};
-    L.p_sub = p_sub;
-    L.npairs = (sigma + 1) / 2;
-    L.ring_base = acols * L.npairs;
-    L.nregions = std::min(kPnMaxRegions, (512 - L.ring_base) / kPnRegionCols);
-    int rows = p_sub + 16;
-    while (rows % 8 != 1) ++rows;
-    L.rows = rows;
-    L.lbo = (uint32_t)rows * 16u;
-    const uint32_t ps = (uint32_t)p_sub, nr = (uint32_t)rows;
-    uint32_t off = 0;
-    L.s_off = off;                    // [step parity] B buffers, 8 * lbo bytes each
-    off += 2u * 8u * L.lbo;
-    L.sym_off = off;                  // [buf][16 steps][p_sub] symbols
-    off += 2u * kPnBlk * ps;
-    L.hdr_off = pn_align16(off);      // [buf][p_sub] headers
-    off = L.hdr_off + 2u * ps * (uint32_t)sizeof(PnHdr);
-    L.rec_off = pn_align16(off);      // [step & 3][rows] uint2 records
-    off = L.rec_off + 4u * nr * 8u;
-    L.xmax_off = pn_align16(off);     // [step parity][rows] float2: max|s| of each half
-    off = L.xmax_off + 2u * nr * 8u;
-    L.fin_off = off;                  // [step parity][p_sub] float2: accept-weighted halves
-    off += 2u * ps * 8u;
-    L.fine_off = off;                 // [step parity][p_sub] int32: final exponent sums
-    off += 2u * ps * 4u;
-    L.e_off = off;                    // [p_sub] int32: exponent sums
-    off += ps * 4u;
-    L.chunk_off = pn_align16(off);    // [step & 3][kPnMaxChunks]
-    off = L.chunk_off + 4u * kPnMaxChunks * (uint32_t)sizeof(PnChunk);
-    L.slot_off = pn_align16(off);     // [p_sub]
-    off = L.slot_off + ps * (uint32_t)sizeof(PnSlot);
-    L.misc_off = pn_align16(off);
-    off = L.misc_off + kPnMiscBytes;
-    L.total = pn_align16(off);
-    return L;
-}
-
-// misc region (bytes, relative to misc_off)
-constexpr uint32_t kMTmem = 0, kMAbort = 4, kMPlanOk = 8, kMFinal = 12,
-                   kMNch = 16,        // int32 [step & 3]
-                   kMBlkAct = 32,     // int32 [buf][loader warp]
-                   kMBar = 64,        // mbarriers, 8 bytes each
-                   kMCnt = 320,       // int32 [16 pairs][2 parities]
-                   kMPinfo = 448,     // int32 [16 pairs][base, neven]
-                   kMRsym = 576,      // float [32]
-                   kMStart = 704,     // uint4 [8]
-                   kMAcc = 832;       // float [64]
-// mbarrier indices
-constexpr int kBarPlan1 = 0,     // [step & 3]   layout, chunk list, records   1 arrival
-              kBarPlan2 = 4,     // [step & 1]   start rows                    1 arrival
-              kBarEpi = 6,       // [step & 3]   epilogue done                 8 arrivals
-              kBarFull = 10,     // [region]     tcgen05.commit
-              kBarEmpty = 16,    // [region]     4 arrivals (the set that drained it)
-              kBarLoaded = 22,   // [buf]        2 arrivals
-              kBarConsumed = 24, // [buf]        1 arrival
-              kBarCount = 26;
-// record of a row (one string at one step): x = destination row * 16 (or kRecFinish | slot),
-// y = slot | kRecFresh
-constexpr uint32_t kRecFresh = 1u << 31;
-
-struct PnParams {
-    const uint8_t *data;
-    int64_t total_bytes;
-    const int64_t *offsets;
-    int64_t n;
-    const uint32_t *tpack;     // [npairs][128][32] 16-bit pairs
-    const float *rsym;         // [sigma] growth bound per symbol
-    const uint4 *start_img;    // [8] start vector, 16-bit, one B row
-    const float *acc;          // [64] accept weights
-    float start_max;
-    int boolean;               // Boolean NFA: threshold every product to {0, 1}, no rescale
-    int kcols;                 // 16-byte core-matrix columns of a B row: 8 (16-bit), 4 (int8)
-    long long wait_cycles;     // limit of one hand-off wait
-    int resc;                  // steps between rescales (power-of-two scaling is exact, so only
-                               // the range matters: 4 for BF16 with growth <= 16 a step, else 1)
-    double ll_empty;
-    int sigma;
-    double *loglik;
-    uint8_t *accept;
-    int32_t *accept_i32;
-    unsigned long long *queue;
-    uint32_t *err;
-    PnLayout L;
-};
 
 // ---- small device helpers -------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pn_smem_u32(const void *p) {
@@ -241,46 +66,14 @@ __device__ __forceinline__ bool pn_mbar_test(uint32_t addr, uint32_t parity) {
         : "=r"(done) : "r"(addr), "r"(parity) : "memory");
     return done != 0;
 }
-// non-suspending test: a spinning waiter sees the phase flip at once (try_wait may park the
-// thread for a few thousand cycles)
-__device__ __forceinline__ bool pn_mbar_poll(uint32_t addr, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    return done != 0;
-}
 __device__ __forceinline__ void pn_mbar_arrive(uint32_t addr) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(addr) : "memory");
 }
 
-// Waits (lane 0 of the calling warp) for the completion of the phase with the
-// given parity; bounded; the result is broadcast to the warp. Spins on the
-// non-suspending test: the hand-offs of this kernel are on its critical path.
-__device__ __forceinline__ bool pn_wait(uint32_t addr, uint32_t parity, volatile uint32_t *abort_flag,
-                                        uint32_t *err, long long limit) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) {
-        const long long t0 = clock64();
-        while (!pn_mbar_poll(addr, parity)) {
-            if (*abort_flag) { ok = 0; break; }
-            if (clock64() - t0 > limit) {
-                atomicOr(err, kPnErrTimeout);
-                *abort_flag = 1u;
-                ok = 0;
-                break;
-            }
-        }
-    }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
-}
-
-// pn_wait with the suspending test: a thread whose phase is not complete may be parked by the
-// hardware instead of spinning, which leaves the issue slots to the warps with work (the lane
-// kernel, whose warps wait a large share of each step)
+// Waits (lane 0 of the calling warp) for the completion of the phase with the given parity;
+// bounded; the result is broadcast to the warp. A thread whose phase is not complete may be
+// parked by the hardware (try_wait) instead of spinning, which leaves the issue slots to the
+// warps with work.
 __device__ __forceinline__ bool pn_wait_park(uint32_t addr, uint32_t parity, volatile uint32_t *abort_flag,
                                              uint32_t *err, long long limit) {
     int ok = 1;
@@ -325,30 +118,6 @@ __device__ __forceinline__ uint16_t pn_to16(float v) {
     else return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
-__device__ __forceinline__ void pn_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// 16 TMEM lanes x 16 columns: thread t gets lanes base + t/4 and base + t/4 + 8 for columns
-// 2(t%4), 2(t%4)+1 and 8 + 2(t%4), 9 + 2(t%4):
-// r = {(l, c), (l, c+1), (l+8, c), (l+8, c+1), (l, c+8), (l, c+9), (l+8, c+8), (l+8, c+9)}.
-__device__ __forceinline__ void pn_tmem_ld16x256(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void pn_tmem_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // two values rounded to the operand type, packed low/high
 template <bool FP16>
 __device__ __forceinline__ uint32_t pn_pack2(float lo, float hi) {
@@ -361,18 +130,6 @@ __device__ __forceinline__ uint32_t pn_pack2(float lo, float hi) {
     }
 }
 
-__device__ __forceinline__ void pn_tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-        "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-           "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-           "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-           "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-           "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
-
 __device__ __forceinline__ void pn_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
@@ -383,711 +140,7 @@ __device__ __forceinline__ void pn_tmem_st16(uint32_t taddr, const uint32_t (&r)
         : "memory");
 }
 
-// ---- shared-memory view -------------------------------------------------------------------------
-struct PnShared {
-    uint8_t *base;
-    PnLayout L;
-    __device__ uint8_t *misc() const { return base + L.misc_off; }
-    __device__ volatile uint32_t *u32(uint32_t off) const {
-        return reinterpret_cast<volatile uint32_t *>(misc() + off);
-    }
-    __device__ uint32_t bar(int i) const { return pn_smem_u32(misc() + kMBar + 8 * i); }
-    __device__ uint32_t sbuf(int par) const { return L.s_off + (uint32_t)par * 8u * L.lbo; }
-    __device__ uint8_t *sym(int buf) const { return base + L.sym_off + buf * kPnBlk * L.p_sub; }
-    __device__ PnHdr *hdr(int buf) const {
-        return reinterpret_cast<PnHdr *>(base + L.hdr_off) + buf * L.p_sub;
-    }
-    __device__ uint2 *rec(int s) const {
-        return reinterpret_cast<uint2 *>(base + L.rec_off) + (s & 3) * L.rows;
-    }
-    __device__ float2 *xmax(int s) const {
-        return reinterpret_cast<float2 *>(base + L.xmax_off) + (s & 1) * L.rows;
-    }
-    __device__ float2 *fin(int s) const {
-        return reinterpret_cast<float2 *>(base + L.fin_off) + (s & 1) * L.p_sub;
-    }
-    __device__ int32_t *finE(int s) const {
-        return reinterpret_cast<int32_t *>(base + L.fine_off) + (s & 1) * L.p_sub;
-    }
-    __device__ int32_t *E() const { return reinterpret_cast<int32_t *>(base + L.e_off); }
-    __device__ PnChunk *chunks(int s) const {
-        return reinterpret_cast<PnChunk *>(base + L.chunk_off) + (s & 3) * kPnMaxChunks;
-    }
-    __device__ PnSlot *slots() const { return reinterpret_cast<PnSlot *>(base + L.slot_off); }
-    __device__ volatile int32_t *nch(int s) const {
-        return reinterpret_cast<volatile int32_t *>(misc() + kMNch) + (s & 3);
-    }
-    __device__ int32_t *cnt() const { return reinterpret_cast<int32_t *>(misc() + kMCnt); }
-    __device__ int32_t *pinfo() const { return reinterpret_cast<int32_t *>(misc() + kMPinfo); }
-};
-
-// phase parity of the k-th completion of a barrier that completes once every `period` steps
-__device__ __forceinline__ uint32_t pn_par(int step, int period) { return (uint32_t)(step / period) & 1u; }
-
-// ---- loader: warps 13-14 -------------------------------------------------------------------------
-__device__ void pn_loader(const PnParams &P, const PnShared &S, volatile uint32_t *abort_flag) {
-    const int lane = threadIdx.x & 31;
-    const int lw = (threadIdx.x >> 5) - kPnLoadWarp0;
-    const int ll = lw * 32 + lane;
-    const int PC = S.L.p_sub;
-    const uint32_t sig4 = (uint32_t)P.sigma * 0x01010101u;
-    int32_t seq[8];
-    int64_t pos[8], end[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { seq[i] = -1; pos[i] = 0; end[i] = 0; }
-    for (int blk = 0;; ++blk) {
-        const int buf = blk & 1;
-        if (blk >= 2 && !pn_wait(S.bar(kBarConsumed + buf), (uint32_t)((blk - 2) >> 1) & 1u,
-                                 abort_flag, P.err, P.wait_cycles))
-            break;
-        uint8_t *sym = S.sym(buf);
-        PnHdr *hd = S.hdr(buf);
-        int nact = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int j = ll + 64 * i;
-            if (j >= PC) continue;
-            uint8_t flags = 0;
-            if (seq[i] < 0 || pos[i] >= end[i]) {
-                seq[i] = -1;
-                for (;;) {
-                    const unsigned long long idx = atomicAdd(P.queue, 1ull);
-                    if (idx >= (unsigned long long)P.n) break;
-                    int64_t p0 = P.offsets[idx], p1 = P.offsets[idx + 1];
-                    if (p0 < 0 || p1 < p0 || p1 > P.total_bytes) {
-                        atomicOr(P.err, kPnErrOffsets);
-                        continue;
-                    }
-                    while (p0 < p1 && P.data[p0] >= (uint8_t)P.sigma) ++p0;
-                    if (p0 == p1) {
-                        pn_write_result(P.loglik, P.accept, P.accept_i32, (int64_t)idx, P.ll_empty);
-                        continue;
-                    }
-                    seq[i] = (int32_t)idx;
-                    pos[i] = p0;
-                    end[i] = p1;
-                    flags = kHdrStart;
-                    break;
-                }
-            }
-            int count = 0;
-            if (seq[i] >= 0) {
-                int64_t p = pos[i];
-                const int64_t e = end[i];
-                bool fast = false;
-                // 20-byte window of aligned words; only when it lies inside [data, data + e)
-                const uintptr_t ap = reinterpret_cast<uintptr_t>(P.data + p);
-                const uintptr_t aw = ap & ~(uintptr_t)3;
-                if (e - p >= 20 && aw >= reinterpret_cast<uintptr_t>(P.data)) {
-                    const uint32_t *wp = reinterpret_cast<const uint32_t *>(aw);
-                    uint32_t w[5];
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) w[k] = __ldg(wp + k);
-                    const uint32_t sh = (uint32_t)(ap & 3) * 8u;
-                    uint32_t wd[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) wd[k] = __funnelshift_r(w[k], w[k + 1], sh);
-                    uint32_t bad = 0;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) bad |= __vcmpgeu4(wd[k], sig4);
-                    if (bad == 0) {
-                        fast = true;
-#pragma unroll
-                        for (int s = 0; s < 16; ++s)
-                            sym[s * PC + j] = (uint8_t)(wd[s >> 2] >> (8 * (s & 3)));
-                        count = 16;
-                        p += 16;
-                    }
-                }
-                if (!fast) {
-                    while (count < 16 && p < e) {
-                        const uint8_t b = P.data[p++];
-                        if (b < (uint8_t)P.sigma) sym[(count++) * PC + j] = b;
-                    }
-                }
-                while (p < e && P.data[p] >= (uint8_t)P.sigma) ++p;
-                pos[i] = p;
-                if (p == e) flags |= kHdrEnd;
-            }
-            PnHdr h;
-            h.seq = seq[i];
-            h.count = (uint8_t)count;
-            h.flags = count > 0 ? flags : 0;
-            h.pad = 0;
-            hd[j] = h;
-            nact += count > 0;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nact += __shfl_xor_sync(0xffffffffu, nact, o);
-        if (lane == 0) {
-            reinterpret_cast<volatile int32_t *>(S.misc() + kMBlkAct)[buf * 2 + lw] = nact;
-            pn_mbar_arrive(S.bar(kBarLoaded + buf));
-        }
-        __syncwarp();
-        // both loader warps have written the block: its active count decides the end
-        if (!pn_wait(S.bar(kBarLoaded + buf), (uint32_t)(blk >> 1) & 1u, abort_flag, P.err, P.wait_cycles)) break;
-        const volatile int32_t *ba = reinterpret_cast<const volatile int32_t *>(S.misc() + kMBlkAct);
-        if (ba[buf * 2] + ba[buf * 2 + 1] == 0) break;
-    }
-}
-
-// ---- planner: warps 9-12 ---------------------------------------------------------------------------
-// named barrier 1: the four planner warps only; only warp 9 waits on mbarriers
-__device__ __forceinline__ void pn_plan_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// Per step s, in order:
-//  stage 1 (waits for the symbol block and for the epilogue of step s-4, the last user of the
-//          4-deep record and chunk rings): ranks of the slots by symbol pair, the chunk list of
-//          step s, the records of step s-1 (destination rows); signals kBarPlan1[s & 3].
-//  stage 2 (waits for the epilogue of step s-2): log-likelihoods of the strings that ended at
-//          step s-2, the start vector into the rows of strings that begin at step s (B buffer
-//          s & 1, last read by the MMA of step s-2); signals kBarPlan2[s & 1].
-__device__ void pn_planner(const PnParams &P, const PnShared &S, volatile uint32_t *abort_flag) {
-    const int tid = threadIdx.x - 32 * kPnPlanWarp0;   // 0..127
-    const int lane = tid & 31;
-    const bool leader = tid == 0;
-    const PnLayout &L = S.L;
-    const int PS = L.p_sub;
-    const uint4 *simg = reinterpret_cast<const uint4 *>(S.misc() + kMStart);
-    PnSlot *slots = S.slots();
-    int32_t *cnt = S.cnt();
-    int32_t *pinfo = S.pinfo();
-    volatile uint32_t *plan_ok = S.u32(kMPlanOk);
-    volatile uint32_t *final_flag = S.u32(kMFinal);
-    for (int j = tid; j < PS; j += kPnPlanThreads) {
-        PnSlot z;
-        z.seq = -1; z.pend[0] = -1; z.pend[1] = -1; z.row = 0; z.c = 0; z.flags = 0;
-        z.blkcnt = 0; z.blkflags = 0;
-        slots[j] = z;
-    }
-    for (int k = tid; k < 32; k += kPnPlanThreads) cnt[k] = 0;
-    pn_plan_sync();
-    auto emit = [&](int s_done) {   // strings whose last step was s_done
-        const float2 *fin = S.fin(s_done);
-        const int32_t *finE = S.finE(s_done);
-        for (int j = tid; j < PS; j += kPnPlanThreads) {
-            const int32_t seq = slots[j].pend[s_done & 1];
-            if (seq < 0) continue;
-            const float2 f = fin[j];
-            const double dot = (double)f.x + (double)f.y;
-            const double ll = dot > 0.0 ? log(dot) + (double)finE[j] * 0.69314718055994530942 : -INFINITY;
-            pn_write_result(P.loglik, P.accept, P.accept_i32, seq, ll);
-            slots[j].pend[s_done & 1] = -1;
-        }
-    };
-    for (int s = 0;; ++s) {
-        // ---------------- stage 1 ----------------
-        if (tid < 32) {
-            bool ok = true;
-            if (s >= 4)
-                ok = pn_wait(S.bar(kBarEpi + ((s - 4) & 3)), pn_par(s - 4, 4), abort_flag, P.err, P.wait_cycles);
-            if (ok && s % kPnBlk == 0) {
-                const int blk = s / kPnBlk;
-                if (leader && blk >= 1) pn_mbar_arrive(S.bar(kBarConsumed + ((blk - 1) & 1)));
-                ok = pn_wait(S.bar(kBarLoaded + (blk & 1)), (uint32_t)(blk >> 1) & 1u, abort_flag, P.err, P.wait_cycles);
-                if (ok && leader) {
-                    const volatile int32_t *ba =
-                        reinterpret_cast<const volatile int32_t *>(S.misc() + kMBlkAct);
-                    *final_flag = (ba[(blk & 1) * 2] + ba[(blk & 1) * 2 + 1]) == 0;
-                }
-            }
-            if (leader) *plan_ok = ok ? 1u : 0u;
-        }
-        pn_plan_sync();
-        if (!*plan_ok) return;
-        const int in = s % kPnBlk;
-        const int buf = (s / kPnBlk) & 1;
-        const bool terminal = in == 0 && *final_flag;
-        const uint8_t *sym = S.sym(buf);
-        const PnHdr *hd = S.hdr(buf);
-        int rank[kPnSlotsPerPlanThread], cs[kPnSlotsPerPlanThread], nseq[kPnSlotsPerPlanThread];
-#pragma unroll
-        for (int k = 0; k < kPnSlotsPerPlanThread; ++k) {
-            rank[k] = -1;
-            cs[k] = -1;
-            nseq[k] = -1;
-            const int j = tid + kPnPlanThreads * k;
-            if (j >= PS || terminal) continue;
-            PnSlot sl = slots[j];
-            if (in == 0) {
-                const PnHdr h = hd[j];
-                sl.blkcnt = h.count;
-                sl.blkflags = h.flags;
-                if (h.flags & kHdrStart) nseq[k] = h.seq;
-                slots[j] = sl;
-            }
-            if (in < sl.blkcnt) {
-                const int c = sym[in * PS + j];
-                cs[k] = c;
-                rank[k] = atomicAdd(&cnt[(c >> 1) * 2 + (c & 1)], 1);
-            }
-        }
-        pn_plan_sync();
-        if (tid < 32) {   // pair bases and the chunk list of step s
-            int ne = 0, no = 0;
-            if (lane < L.npairs) {
-                ne = cnt[lane * 2];
-                no = cnt[lane * 2 + 1];
-                cnt[lane * 2] = 0;
-                cnt[lane * 2 + 1] = 0;
-            }
-            const int np = ne + no;
-            const int nc = (np + kPnRegionCols - 1) / kPnRegionCols;
-            int incl = np, cincl = nc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int a = __shfl_up_sync(0xffffffffu, incl, o);
-                const int c = __shfl_up_sync(0xffffffffu, cincl, o);
-                if (lane >= o) { incl += a; cincl += c; }
-            }
-            const int base = incl - np, cbase = cincl - nc;
-            if (lane < L.npairs) {
-                pinfo[lane * 2] = base;
-                pinfo[lane * 2 + 1] = ne;
-                PnChunk *ch = S.chunks(s);
-                for (int k = 0; k < nc; ++k) {
-                    PnChunk d;
-                    d.row0 = (uint16_t)(base + k * kPnRegionCols);
-                    const int cols = min(kPnRegionCols, np - k * kPnRegionCols);
-                    d.ncols = (uint8_t)cols;
-                    d.split = (uint8_t)min(max(ne - k * kPnRegionCols, 0), cols);
-                    d.pair = (uint8_t)lane;
-                    d.pad0 = d.pad1 = d.pad2 = 0;
-                    ch[cbase + k] = d;
-                }
-            }
-            const int total_chunks = __shfl_sync(0xffffffffu, cincl, 31);
-            if (lane == 0) *S.nch(s) = terminal ? kPnTerminate : total_chunks;
-        }
-        pn_plan_sync();
-        uint2 *rec = S.rec(s - 1);
-#pragma unroll
-        for (int k = 0; k < kPnSlotsPerPlanThread; ++k) {
-            const int j = tid + kPnPlanThreads * k;
-            if (j >= PS) continue;
-            PnSlot sl = slots[j];
-            int row1 = -1;
-            if (cs[k] >= 0) {
-                const int p = cs[k] >> 1;
-                row1 = pinfo[p * 2] + ((cs[k] & 1) ? pinfo[p * 2 + 1] : 0) + rank[k];
-            }
-            if (s >= 1 && (sl.flags & kSlotActive)) {
-                uint2 r;
-                r.y = (uint32_t)j | ((sl.flags & kSlotFresh) ? kRecFresh : 0u);
-                if (sl.flags & kSlotLast) {
-                    r.x = kRecFinish | (uint32_t)j;
-                    sl.pend[(s - 1) & 1] = sl.seq;
-                } else {
-                    // a continuing string is active at step s (blocks never leave it empty)
-                    r.x = (uint32_t)max(row1, 0) * 16u;
-                }
-                rec[sl.row] = r;
-            }
-            uint8_t nf = 0;
-            if (nseq[k] >= 0) sl.seq = nseq[k];
-            if (row1 >= 0) {
-                nf |= kSlotActive;
-                if ((sl.blkflags & kHdrEnd) && in == sl.blkcnt - 1) nf |= kSlotLast;
-                if (nseq[k] >= 0) nf |= kSlotFresh;
-                sl.row = (int16_t)row1;
-                sl.c = (uint8_t)cs[k];
-            }
-            sl.flags = nf;
-            slots[j] = sl;
-        }
-        pn_plan_sync();
-        if (leader) pn_mbar_arrive(S.bar(kBarPlan1 + (s & 3)));
-        // ---------------- stage 2 ----------------
-        if (tid < 32) {
-            bool ok = true;
-            if (s >= 2) ok = pn_wait(S.bar(kBarEpi + ((s - 2) & 3)), pn_par(s - 2, 4), abort_flag, P.err, P.wait_cycles);
-            if (leader) *plan_ok = ok ? 1u : 0u;
-        }
-        pn_plan_sync();
-        if (!*plan_ok) return;
-        if (s >= 2) emit(s - 2);
-        if (!terminal) {
-            const uint32_t sb = S.sbuf(s & 1);
-            for (int j = tid; j < PS; j += kPnPlanThreads) {
-                const PnSlot sl = slots[j];
-                if ((sl.flags & kSlotFresh) == 0) continue;
-                uint8_t *dst = S.base + sb + (uint32_t)sl.row * 16u;
-#pragma unroll
-                for (int c = 0; c < P.kcols; ++c) *reinterpret_cast<uint4 *>(dst + c * L.lbo) = simg[c];
-            }
-        }
-        pn_fence_async_smem();
-        pn_plan_sync();
-        if (leader) pn_mbar_arrive(S.bar(kBarPlan2 + (s & 1)));
-        if (terminal) {   // the strings that ended at step s-1, then done
-            if (s >= 1) {
-                if (tid < 32) {
-                    const bool ok = pn_wait(S.bar(kBarEpi + ((s - 1) & 3)), pn_par(s - 1, 4), abort_flag,
-                                            P.err, P.wait_cycles);
-                    if (leader) *plan_ok = ok ? 1u : 0u;
-                }
-                pn_plan_sync();
-                if (*plan_ok) emit(s - 1);
-            }
-            return;
-        }
-    }
-}
-
-// ---- MMA issuer: warp 8 ----------------------------------------------------------------------------
-// KIND: 0 = BF16, 1 = FP16 operands (kind::f16, FP32 sums), 2 = 0/1 int8 operands
-// (kind::i8, unsigned, int32 sums: K = 32 an instruction, half the instructions).
-template <int KIND>
-__device__ void pn_mma(const PnParams &P, const PnShared &S, uint32_t tbase,
-                       volatile uint32_t *abort_flag) {
-    constexpr bool I8 = KIND == 2;
-    constexpr int kKSteps = I8 ? 2 : 4;              // K = 64 as 2 x K32 or 4 x K16
-    constexpr uint32_t kACols = I8 ? 16u : 32u;      // TMEM columns of a pair's A
-    const int lane = threadIdx.x & 31;
-    const PnLayout &L = S.L;
-    const uint32_t fmt = KIND == 1 ? 0u : 1u;
-    const uint32_t smem_base = pn_smem_u32(S.base);
-    const uint32_t desc_hi = (128u >> 4) | (1u << 14);   // SBO = 128 B, descriptor version 1
-    const uint32_t nr = (uint32_t)L.nregions;
-    uint32_t g = 0;
-    for (int t = 0;; ++t) {
-        if (!pn_wait(S.bar(kBarPlan2 + (t & 1)), pn_par(t, 2), abort_flag, P.err, P.wait_cycles)) break;
-        const int nch = *S.nch(t);
-        if (nch == kPnTerminate) break;
-        if (t >= 1 && !pn_wait(S.bar(kBarEpi + ((t - 1) & 3)), pn_par(t - 1, 4), abort_flag, P.err, P.wait_cycles)) break;
-        const PnChunk *ch = S.chunks(t);
-        const uint32_t sb = smem_base + S.sbuf(t & 1);
-        bool aborted = false;
-        for (int k = 0; k < nch; ++k) {
-            const PnChunk d = ch[k];
-            const uint32_t r = g % nr, u = g / nr;
-            if (u > 0 && !pn_wait(S.bar(kBarEmpty + (int)r), (u - 1) & 1u, abort_flag, P.err, P.wait_cycles)) {
-                aborted = true;
-                break;
-            }
-            pn_tc_after();
-            if (lane == 0) {
-                const uint32_t n16 = ((uint32_t)d.ncols + 15u) & ~15u;
-                // instruction descriptor: D format (bits 4-5: F32 = 1, S32 = 2), A and B
-                // formats (bits 7-9, 10-12: F16 = 0 / BF16 = 1; U8 = 0), N / 8 (17-22),
-                // M / 16 (24-28); both operands K-major
-                const uint32_t idesc = I8 ? ((2u << 4) | ((n16 >> 3) << 17) | ((128u >> 4) << 24))
-                                          : ((1u << 4) | (fmt << 7) | (fmt << 10) | ((n16 >> 3) << 17) |
-                                             ((128u >> 4) << 24));
-                const uint32_t td = tbase + (uint32_t)L.ring_base + r * kPnRegionCols;
-                // every K step spans two 16-byte core-matrix columns of B (16 states of
-                // 16 bits, or 32 states of 8 bits) and 8 TMEM columns of A
-#pragma unroll
-                for (int kk = 0; kk < kKSteps; ++kk) {
-                    const uint32_t saddr = sb + (uint32_t)d.row0 * 16u + (uint32_t)kk * 2u * L.lbo;
-                    const uint64_t desc = (uint64_t)(((saddr >> 4) & 0x3FFFu) | ((L.lbo >> 4) << 16)) |
-                                          ((uint64_t)desc_hi << 32);
-                    const uint32_t ta = tbase + kACols * d.pair + 8u * kk;
-                    const uint32_t acc = kk > 0;
-                    if constexpr (I8)
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-                            :: "r"(td), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
-                    else
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                            :: "r"(td), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
-                }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                    :: "r"(S.bar(kBarFull + (int)r)) : "memory");
-            }
-            __syncwarp();
-            ++g;
-        }
-        if (aborted) break;
-    }
-    // Drain: every committed chain must have finished before the TMEM is freed.
-    for (uint32_t r = 0; r < nr && r < g; ++r) {
-        const uint32_t uses = (g - r + nr - 1) / nr;   // commits made to region r
-        if (lane == 0) {                               // completion of the last one
-            const long long t0 = clock64();
-            while (!pn_mbar_test(S.bar(kBarFull + (int)r), (uses - 1) & 1u)) {
-                if (clock64() - t0 > kPnDrainCycles) { atomicOr(P.err, kPnErrTimeout); break; }
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// ---- epilogue: warps 0-7 ---------------------------------------------------------------------------
-// Two sets of four warps take alternate chunks. Warp q of a set reads TMEM lanes 32q..32q+31: the
-// even symbol's states 32(q&1).. for q < 2, the odd symbol's for q >= 2. The A rows are permuted
-// so that in each 16-lane half h the lanes j and j + 8 hold the adjacent states 2j and 2j + 1: a
-// 16x256b load then gives thread t (j = t/4) the states 32(q&1) + 16h + 2j, +1 of four columns,
-// which it scales, packs into one 32-bit store per pair, and reduces (max) with the seven other
-// threads holding the same columns. The scale of a column, 2^-f with f the exponent of
-// max|s_t| * R_c (max|s_t| left by the previous step's epilogue), is computed by one lane per
-// column and shuffled to the others; warps q = 0, 2 keep the exponent sums.
-template <int KIND>
-__device__ void pn_epilogue(const PnParams &P, const PnShared &S, uint32_t tbase,
-                            volatile uint32_t *abort_flag) {
-    constexpr bool I8 = KIND == 2, FP16 = KIND == 1;
-    const int lane = threadIdx.x & 31;
-    const int ew = threadIdx.x >> 5;
-    const int q = ew & 3;                           // TMEM lane quadrant
-    const uint32_t set = (uint32_t)(ew >> 2);       // chunk parity this warp drains
-    const PnLayout &L = S.L;
-    const int j = lane >> 2, cp = lane & 3;
-    const int sg0 = 32 * (q & 1) + 2 * j, sg1 = sg0 + 16;   // first states of the two pairs
-    // byte offsets of states sg0 and sg1 in a B row: 8 states of 16 bits, or 16 of 8 bits, a
-    // core-matrix column
-    const uint32_t toff0 = I8 ? (uint32_t)(sg0 >> 4) * L.lbo + (uint32_t)(sg0 & 15)
-                              : (uint32_t)(sg0 >> 3) * L.lbo + (uint32_t)(sg0 & 7) * 2u;
-    const uint32_t toff1 = I8 ? (uint32_t)(sg1 >> 4) * L.lbo + (uint32_t)(sg1 & 15)
-                              : (uint32_t)(sg1 >> 3) * L.lbo + (uint32_t)(sg1 & 7) * 2u;
-    const float *accv = reinterpret_cast<const float *>(S.misc() + kMAcc);
-    const float a00 = accv[sg0], a01 = accv[sg0 + 1], a10 = accv[sg1], a11 = accv[sg1 + 1];
-    const float *rsym = reinterpret_cast<const float *>(S.misc() + kMRsym);
-    const bool even = q < 2;
-    const bool owner = (q & 1) == 0;
-    const bool bmode = P.boolean != 0;
-    int32_t *E = S.E();
-    const uint32_t nr = (uint32_t)L.nregions;
-    uint32_t g = 0;
-    if (!pn_wait(S.bar(kBarPlan1), 0u, abort_flag, P.err, P.wait_cycles)) return;
-    for (int t = 0;; ++t) {
-        const int nch = *S.nch(t);   // plan of step t: waited for in the previous iteration
-        if (nch == kPnTerminate) break;
-        // records of step t come with the plan of step t+1; the maxima of step t from both sets
-        if (!pn_wait(S.bar(kBarPlan1 + ((t + 1) & 3)), pn_par(t + 1, 4), abort_flag, P.err, P.wait_cycles)) break;
-        if (t >= 1 && !pn_wait(S.bar(kBarEpi + ((t - 1) & 3)), pn_par(t - 1, 4), abort_flag, P.err, P.wait_cycles)) break;
-        const PnChunk *ch = S.chunks(t);
-        const uint2 *rec = S.rec(t);
-        const float2 *xm = S.xmax(t);
-        // a rescale step scales by the maxima that the step before it found
-        const bool scale_step = t % P.resc == 0, max_step = (t + 1) % P.resc == 0;
-        float *xn = reinterpret_cast<float *>(S.xmax(t + 1)) + (q & 1);
-        float *fin = reinterpret_cast<float *>(S.fin(t)) + (q & 1);
-        int32_t *finE = S.finE(t);
-        uint8_t *snext = S.base + S.sbuf((t + 1) & 1);
-        bool aborted = false;
-        for (int k = 0; k < nch; ++k, ++g) {
-            if ((g & 1u) != set) continue;
-            const PnChunk d = ch[k];
-            const uint32_t r = g % nr, u = g / nr;
-            if (!pn_wait(S.bar(kBarFull + (int)r), u & 1u, abort_flag, P.err, P.wait_cycles)) {
-                aborted = true;
-                break;
-            }
-            pn_tc_after();
-            const int c_lo = even ? 0 : d.split;
-            const int c_hi = even ? d.split : d.ncols;
-            const float R = rsym[2 * d.pair + (even ? 0 : 1)];
-            const uint32_t tcol = tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)L.ring_base +
-                                  r * kPnRegionCols;
-            for (int c = c_lo & ~15; c < c_hi; c += 16) {
-                uint32_t v0[8], v1[8];
-                pn_tmem_ld16x256(tcol + (uint32_t)c, v0);
-                pn_tmem_ld16x256(tcol + (16u << 16) + (uint32_t)c, v1);
-                // lane l < 16: the scale of column c + l (and the exponent sum of its string)
-                float scl = 1.f;
-                {
-                    const int col = c + lane;
-                    if (lane < 16 && col >= c_lo && col < c_hi && bmode) {
-                        // Boolean forms: no scaling, the exponent sum stays 0
-                        const uint2 rcl = rec[d.row0 + col];
-                        if (owner && (rcl.x & kRecFinish)) finE[rcl.y & 1023u] = 0;
-                    } else if (lane < 16 && col >= c_lo && col < c_hi && !scale_step) {
-                        // no rescale this step: a string that begins starts its exponent sum
-                        const uint2 rcl = rec[d.row0 + col];
-                        const int jl = (int)(rcl.y & 1023u);
-                        if (owner) {
-                            const int e = (rcl.y & kRecFresh) ? 0 : E[jl];
-                            if (rcl.y & kRecFresh) E[jl] = 0;
-                            if (rcl.x & kRecFinish) finE[jl] = e;
-                        }
-                    } else if (lane < 16 && col >= c_lo && col < c_hi) {
-                        const int row = d.row0 + col;
-                        const uint2 rcl = rec[row];
-                        const bool fresh = (rcl.y & kRecFresh) != 0;
-                        const int jl = (int)(rcl.y & 1023u);
-                        float m;
-                        if (fresh) {
-                            m = P.start_max;
-                        } else {
-                            const float2 x2 = xm[row];
-                            m = fmaxf(x2.x, x2.y);
-                        }
-                        int f = pn_ceil_exp(m * R);
-                        f = min(max(f, -125), 125);
-                        scl = pn_pow2(-f);
-                        if (owner) {
-                            const int e = (fresh ? 0 : E[jl]) + f;
-                            E[jl] = e;
-                            if (rcl.x & kRecFinish) finE[jl] = e;
-                        }
-                    }
-                }
-                // this thread's columns: c + {2cp, 2cp+1, 2cp+8, 2cp+9}
-                uint2 rc[4];
-                bool valid[4];
-                float sc[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int co = (i >> 1) * 8 + 2 * cp + (i & 1);
-                    const int col = c + co;
-                    valid[i] = col >= c_lo && col < c_hi;
-                    rc[i] = rec[d.row0 + (valid[i] ? col : c_lo)];
-                    sc[i] = __shfl_sync(0xffffffffu, scl, co);
-                }
-                pn_tmem_wait_ld();
-                float x[4][4], m[4];
-                bool any_fin = false;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int ri = (i >> 1) * 4 + (i & 1);
-                    if constexpr (I8) {   // int32 path counts: reachable when nonzero
-                        x[i][0] = v0[ri] != 0u ? 1.f : 0.f;
-                        x[i][1] = v0[ri + 2] != 0u ? 1.f : 0.f;
-                        x[i][2] = v1[ri] != 0u ? 1.f : 0.f;
-                        x[i][3] = v1[ri + 2] != 0u ? 1.f : 0.f;
-                    } else {
-                        x[i][0] = __uint_as_float(v0[ri]) * sc[i];       // state sg0
-                        x[i][1] = __uint_as_float(v0[ri + 2]) * sc[i];   // sg0 + 1
-                        x[i][2] = __uint_as_float(v1[ri]) * sc[i];       // sg1
-                        x[i][3] = __uint_as_float(v1[ri + 2]) * sc[i];   // sg1 + 1
-                    }
-                    if (!I8 && bmode) {   // reachability: exact, the sums are small integers
-#pragma unroll
-                        for (int z = 0; z < 4; ++z) x[i][z] = x[i][z] > 0.f ? 1.f : 0.f;
-                    }
-                    const bool fin_i = (rc[i].x & kRecFinish) != 0;
-                    const bool keep = valid[i] && !fin_i;
-                    any_fin |= valid[i] && fin_i;
-                    if (keep) {
-                        uint8_t *dst = snext + rc[i].x;
-                        if constexpr (I8) {   // two adjacent states, one byte each
-                            *reinterpret_cast<uint16_t *>(dst + toff0) =
-                                (uint16_t)((x[i][0] != 0.f ? 1u : 0u) | (x[i][1] != 0.f ? 0x100u : 0u));
-                            *reinterpret_cast<uint16_t *>(dst + toff1) =
-                                (uint16_t)((x[i][2] != 0.f ? 1u : 0u) | (x[i][3] != 0.f ? 0x100u : 0u));
-                        } else {
-                            *reinterpret_cast<uint32_t *>(dst + toff0) = pn_pack2<FP16>(x[i][0], x[i][1]);
-                            *reinterpret_cast<uint32_t *>(dst + toff1) = pn_pack2<FP16>(x[i][2], x[i][3]);
-                        }
-                    }
-                    m[i] = keep ? fmaxf(fmaxf(fabsf(x[i][0]), fabsf(x[i][1])),
-                                        fmaxf(fabsf(x[i][2]), fabsf(x[i][3])))
-                                : 0.f;
-                }
-                // column maxima over this warp's 32 states: the 8 threads with the same cp
-                // (they set the next rescale step's scale; the Boolean forms do not scale)
-                if (!bmode && max_step) {
-#pragma unroll
-                    for (int o = 4; o < 32; o <<= 1)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
-                    if (j == 0) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (valid[i] && !(rc[i].x & kRecFinish)) xn[(rc[i].x >> 4) * 2] = m[i];
-                    }
-                }
-                if (__any_sync(0xffffffffu, any_fin)) {   // last symbols: accept-weighted sums
-                    float pz[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        pz[i] = x[i][0] * a00 + x[i][1] * a01 + x[i][2] * a10 + x[i][3] * a11;
-#pragma unroll
-                    for (int o = 4; o < 32; o <<= 1)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) pz[i] += __shfl_xor_sync(0xffffffffu, pz[i], o);
-                    if (j == 0) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (valid[i] && (rc[i].x & kRecFinish)) fin[(rc[i].x & 1023u) * 2] = pz[i];
-                    }
-                }
-            }
-            pn_tc_before();
-            __syncwarp();
-            if (lane == 0) pn_mbar_arrive(S.bar(kBarEmpty + (int)r));
-        }
-        if (aborted) break;
-        pn_fence_async_smem();
-        __syncwarp();
-        if (lane == 0) pn_mbar_arrive(S.bar(kBarEpi + (t & 3)));
-    }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(kPnThreads, 1) pnfa_tc_kernel(PnParams P) {
-    extern __shared__ __align__(1024) uint8_t pn_smem[];
-    PnShared S{pn_smem, P.L};
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *misc = S.misc();
-    for (int i = threadIdx.x; i < kPnMiscBytes / 4; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(misc)[i] = 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kBarCount; ++i) {
-            uint32_t count = 1;
-            if (i >= kBarEpi && i < kBarEpi + 4)
-                count = kPnEpiWarps;
-            else if (i >= kBarEmpty && i < kBarEmpty + kPnMaxRegions)
-                count = 4;
-            else if (i >= kBarLoaded && i < kBarLoaded + 2)
-                count = kPnLoadWarps;
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(S.bar(i)), "r"(count));
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (threadIdx.x < P.sigma) reinterpret_cast<float *>(misc + kMRsym)[threadIdx.x] = P.rsym[threadIdx.x];
-    if (threadIdx.x < 8) reinterpret_cast<uint4 *>(misc + kMStart)[threadIdx.x] = P.start_img[threadIdx.x];
-    if (threadIdx.x < 64) reinterpret_cast<float *>(misc + kMAcc)[threadIdx.x] = P.acc[threadIdx.x];
-    if (warp == kPnMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(pn_smem_u32(misc + kMTmem)), "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    pn_tc_before();
-    __syncthreads();
-    pn_tc_after();
-    const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(misc + kMTmem);
-    // A operands: pair p -> TMEM columns [32p, 32p + 32) (16-bit values, two a column) or
-    // [16p, 16p + 16) (int8, four a column), lane = row of [T[2p]; T[2p+1]]
-    if (warp < 4) {
-        for (int p = 0; p < P.L.npairs; ++p) {
-            if constexpr (KIND == 2) {
-                const uint32_t *src = P.tpack + ((size_t)p * 128 + 32 * warp + lane) * 16;
-                uint32_t r[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) r[k] = __ldg(src + k);
-                pn_tmem_st16(tbase + ((uint32_t)(32 * warp) << 16) + 16u * p, r);
-            } else {
-                const uint32_t *src = P.tpack + ((size_t)p * 128 + 32 * warp + lane) * 32;
-                uint32_t r[32];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) r[k] = __ldg(src + k);
-                pn_tmem_st32(tbase + ((uint32_t)(32 * warp) << 16) + 32u * p, r);
-            }
-        }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    }
-    pn_tc_before();
-    __syncthreads();
-    pn_tc_after();
-    volatile uint32_t *abort_flag = S.u32(kMAbort);
-    if (warp < kPnEpiWarps) pn_epilogue<KIND>(P, S, tbase, abort_flag);
-    else if (warp == kPnMmaWarp) pn_mma<KIND>(P, S, tbase, abort_flag);
-    else if (warp < kPnLoadWarp0) pn_planner(P, S, abort_flag);
-    else pn_loader(P, S, abort_flag);
-    pn_tc_before();
-    __syncthreads();
-    pn_tc_after();
-    if (warp == kPnMmaWarp)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(512));
-}
-
-// ---- strings on TMEM lanes (alphabets of at most two symbols) -------------------------------
+// ---- strings on TMEM lanes (alphabets of at most four symbols) -------------------------------
 // Each of four tiles of 128 strings keeps one string on each TMEM lane: the string's state is
 // row m of the tile's A operand, K = 64 * sigma, with the 64 states in the K range of the
 // string's next symbol and zeros in the other range; B (shared memory) stacks the tables,
@@ -1781,16 +834,16 @@ pnfa_chain_kernel(PnPlainParams P, const uint16_t *T16, int resc) {
 }  // namespace trex
 
 #include "pnfa_fp32.cuh"
+#include "pnfa_sym.cuh"
 
 // ---- handle -----------------------------------------------------------------------------------
 struct trex_pnfa {
-    int n_states = 0, sigma = 0, npairs = 0, n_sms = 0;
+    int n_states = 0, sigma = 0, n_sms = 0;
     double ll_empty = 0.0, ll_empty_bool = 0.0;
     // tensor-core tables: [bf16, fp16, Boolean 0/1 in bf16, Boolean 0/1 in int8]
     float start_max16[4] = {0.f, 0.f, 0.f, 0.f};
     float *d_T32 = nullptr, *d_start32 = nullptr, *d_acc = nullptr, *d_acc_bool = nullptr;
     uint16_t *d_T16[2] = {nullptr, nullptr};   // [sigma][64][64] row-major: bf16, fp16
-    uint32_t *d_tpack[4] = {nullptr, nullptr, nullptr, nullptr};
     float *d_rsym[4] = {nullptr, nullptr, nullptr, nullptr};
     uint4 *d_simg[4] = {nullptr, nullptr, nullptr, nullptr};
     uint8_t *d_misc = nullptr;   // [0,8) queue, [8,12) error word
@@ -1825,7 +878,6 @@ static void pn_free(trex_pnfa *h) {
     cudaFree(h->d_acc);
     cudaFree(h->d_acc_bool);
     for (int k = 0; k < 4; ++k) {
-        cudaFree(h->d_tpack[k]);
         cudaFree(h->d_rsym[k]);
         cudaFree(h->d_simg[k]);
     }
@@ -1838,45 +890,27 @@ static int64_t pn_sms(const trex_pnfa *h) {
 
 // Tables, rings, slots and shared-memory layout of a run of pnfa_fp32_kernel: one CTA an SM, the
 // strings spread over all SMs, as many slots a CTA as it has strings or fit beside the tables.
-static SyParams sy_params(const trex_pnfa *h, int64_t n) {
-    SyParams Q{};
+static RiParams ri_params(const trex_pnfa *h, int64_t n) {
+    RiParams Q{};
     Q.T32 = h->d_T32;
     Q.start_img = reinterpret_cast<const uint4 *>(h->d_start32);
     Q.acc = h->d_acc;
     Q.ll_empty = h->ll_empty;
     Q.wait_cycles = mbar_wait_cycles();
     Q.sigma = h->sigma;
-    Q.rep = std::max(1, kSyWarps / h->sigma);
+    Q.rep = std::max(1, kRiWarps / h->sigma);
     Q.n_rings = Q.sigma * Q.rep;
     Q.grid = (int)std::max<int64_t>(1, std::min<int64_t>(n, pn_sms(h)));
-    Q.slots = (int)std::min<int64_t>((n + Q.grid - 1) / Q.grid, kSyMaxSlots);
+    Q.slots = (int)std::min<int64_t>((n + Q.grid - 1) / Q.grid, kRiMaxSlots);
     for (;; --Q.slots) {
         Q.rep_shift = 5;
         while ((1 << Q.rep_shift) < Q.slots) ++Q.rep_shift;
         Q.ring_cap = 1 << Q.rep_shift;
-        Q.recs_off = pn_align16(kSyRings + (uint32_t)(Q.n_rings + 1) * (uint32_t)Q.ring_cap * 2u);
-        Q.rows_off = Q.recs_off + (uint32_t)Q.slots * kSyRecBytes;
-        Q.tbl_off = Q.rows_off + (uint32_t)Q.slots * kSyRowBytes;
-        if (Q.tbl_off + (uint32_t)Q.sigma * kSyTblBytes <= kPnSmemCap) return Q;
+        Q.recs_off = pn_align16(kRiRings + (uint32_t)(Q.n_rings + 1) * (uint32_t)Q.ring_cap * 2u);
+        Q.rows_off = Q.recs_off + (uint32_t)Q.slots * kRiRecBytes;
+        Q.tbl_off = Q.rows_off + (uint32_t)Q.slots * kRiRowBytes;
+        if (Q.tbl_off + (uint32_t)Q.sigma * kRiTblBytes <= kPnSmemCap) return Q;
     }
-}
-
-static int pn_choose(const trex_pnfa *h, int64_t n, int *grid, int *p_sub) {
-    int pmax = 0;
-    for (int p = 32; p <= kPnMaxPSub; p += 32)
-        if (pn_layout(p, h->sigma).total <= kPnSmemCap) pmax = p;
-    if (pmax == 0) return TREX_ERR_SHAPE;
-    const int64_t sms = pn_sms(h);
-    if (n <= sms * 64) {
-        *grid = (int)std::max<int64_t>(1, (n + 63) / 64);
-        *p_sub = 64;
-    } else {
-        *grid = (int)sms;
-        int64_t need = (n + sms - 1) / sms;
-        need = (need + 31) / 32 * 32;
-        *p_sub = (int)std::min<int64_t>(need, pmax);
-    }
-    return TREX_OK;
 }
 
 }  // namespace trex
@@ -1894,7 +928,6 @@ int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start
     if (!h) return TREX_ERR_OOM;
     h->n_states = n_states;
     h->sigma = sigma;
-    h->npairs = (sigma + 1) / 2;
     h->n_sms = sm_count();
     if (h->n_sms <= 0) {
         delete h;
@@ -1924,30 +957,19 @@ int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start
         nacc += sb[i] != 0.f && ab[i] != 0.f;
     }
     h->ll_empty_bool = nacc ? std::log((double)nacc) : -INFINITY;
-    std::vector<uint32_t> tp[4];
     std::vector<float> rs[4];
     std::vector<uint4> simg[4];
     for (int k = 0; k < 3; ++k) {
         const bool fp16 = k == 1;
         const std::vector<float> &Tk = k == 2 ? Tb : T32;
         const std::vector<float> &sk = k == 2 ? sb : s32;
-        tp[k].assign((size_t)h->npairs * 128 * 32, 0u);
         rs[k].assign(sigma, 0.f);
         for (int c = 0; c < sigma; ++c) {
-            const int p = c >> 1, half_ = c & 1;
             double rmax = 0.0;
-            for (int rr = 0; rr < 64; ++rr) {
-                // A row rr holds destination state d: in each group of 16 rows, rows 0-7 are the
-                // even states and rows 8-15 the odd ones, so TMEM lanes j and j+8 of a 16-lane
-                // half carry the adjacent states 2j and 2j+1 (the epilogue's 16x256b loads)
-                const int d = (rr & ~15) | ((rr & 7) << 1) | ((rr >> 3) & 1);
+            for (int d = 0; d < 64; ++d) {
                 double rsum = 0.0;
-                for (int q = 0; q < 64; ++q) {
-                    const uint16_t v = pn_host16(Tk[((size_t)c * 64 + d) * 64 + q], fp16);
-                    rsum += std::fabs((double)pn_host16_to_f(v, fp16));
-                    uint32_t &w = tp[k][((size_t)p * 128 + half_ * 64 + rr) * 32 + (q >> 1)];
-                    w |= (uint32_t)v << (16 * (q & 1));
-                }
+                for (int q = 0; q < 64; ++q)
+                    rsum += std::fabs((double)pn_host16_to_f(pn_host16(Tk[((size_t)c * 64 + d) * 64 + q], fp16), fp16));
                 rmax = std::max(rmax, rsum);
             }
             // a little above the largest row sum: bounds max|T s| / max|s| through FP32 rounding
@@ -1969,21 +991,11 @@ int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start
             if (k == 0) h->tc_resc = h->chain_resc[0];
         }
     }
-    {   // int8 Boolean tables: the same A rows as above with 0/1 bytes, four K values a word
-        tp[3].assign((size_t)h->npairs * 128 * 16, 0u);
-        for (int c = 0; c < sigma; ++c) {
-            const int p = c >> 1, half_ = c & 1;
-            for (int rr = 0; rr < 64; ++rr) {
-                const int d = (rr & ~15) | ((rr & 7) << 1) | ((rr >> 3) & 1);
-                for (int q = 0; q < 64; ++q)
-                    if (Tb[((size_t)c * 64 + d) * 64 + q] != 0.f)
-                        tp[3][((size_t)p * 128 + half_ * 64 + rr) * 16 + (q >> 2)] |= 1u << (8 * (q & 3));
-            }
-        }
+    {   // int8 Boolean form
         rs[3] = rs[2];
-        simg[3].assign(8, make_uint4(0, 0, 0, 0));   // a B row: 16 states a 16-byte column
+        simg[3].assign(8, make_uint4(0, 0, 0, 0));   // a state row of bytes
         uint8_t *b = reinterpret_cast<uint8_t *>(simg[3].data());
-        for (int i = 0; i < 64; ++i) b[(i >> 4) * 16 + (i & 15)] = sb[i] != 0.f ? 1 : 0;
+        for (int i = 0; i < 64; ++i) b[i] = sb[i] != 0.f ? 1 : 0;
         h->start_max16[3] = 1.f;
     }
     cudaError_t e = cudaSuccess;
@@ -2002,29 +1014,19 @@ int trex_pnfa_create(int n_states, int sigma, const float *T, const float *start
     up((void **)&h->d_acc, a32.data(), 256);
     up((void **)&h->d_acc_bool, ab.data(), 256);
     for (int k = 0; k < 4; ++k) {
-        up((void **)&h->d_tpack[k], tp[k].data(), tp[k].size() * 4);
         up((void **)&h->d_rsym[k], rs[k].data(), rs[k].size() * 4);
         up((void **)&h->d_simg[k], simg[k].data(), 8 * sizeof(uint4));
     }
     if (e == cudaSuccess) e = cudaMalloc(&h->d_misc, 16);
     if (e == cudaSuccess) e = cudaMemset(h->d_misc, 0, 16);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPnSmemCap);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPnSmemCap);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPnSmemCap);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPnSmemCap);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_chain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPnSmemCap);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pnfa_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPnSmemCap);
+    // the attribute is per kernel: raised to what any handle can need
+    for (const void *f :
+         {(const void *)pnfa_sym_kernel<0, false>, (const void *)pnfa_sym_kernel<0, true>,
+          (const void *)pnfa_sym_kernel<1, false>, (const void *)pnfa_sym_kernel<1, true>,
+          (const void *)pnfa_sym_kernel<2, false>, (const void *)pnfa_sym_kernel<2, true>,
+          (const void *)pnfa_sym_kernel<3, false>, (const void *)pnfa_sym_kernel<3, true>,
+          (const void *)pnfa_fp32_kernel, (const void *)pnfa_chain_kernel<false>, (const void *)pnfa_chain_kernel<true>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPnSmemCap);
     if (e != cudaSuccess) {
         set_last_error("trex_pnfa_create", e);
         pn_free(h);
@@ -2093,8 +1095,8 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
         }
         // alphabets whose tables fit on an SM: strings in rings by symbol (8192 strings x 512, 20
         // symbols: 1.73 ms against 16.7); larger ones read every table through L1 and L2
-        if (h->sigma <= kSyWarps) {
-            SyParams S = sy_params(h, n_strings);
+        if (h->sigma <= kRiWarps) {
+            RiParams S = ri_params(h, n_strings);
             S.data = data;
             S.total_bytes = total_bytes;
             S.offsets = offsets;
@@ -2105,7 +1107,7 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
             S.queue = queue;
             S.err = err;
             profile_kernel_begin(st);
-            pnfa_fp32_kernel<<<S.grid, 32 * S.n_rings, S.tbl_off + (uint32_t)S.sigma * kSyTblBytes, st>>>(S);
+            pnfa_fp32_kernel<<<S.grid, 32 * S.n_rings, S.tbl_off + (uint32_t)S.sigma * kRiTblBytes, st>>>(S);
             profile_kernel_end(st);
             TREX_CHECK_LAUNCH();
             return TREX_OK;
@@ -2154,42 +1156,56 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
         TREX_CHECK_LAUNCH();
         return TREX_OK;
     }
-    if (h->sigma > kPnMaxSigmaTc) {
+    if (h->sigma > kSyMaxSigma) {
         set_last_error_msg("trex_pnfa_run: the tensor-core form takes at most 28 symbols");
         return TREX_ERR_SHAPE;
     }
-    int grid = 0, p_sub = 0;
-    int rc = pn_choose(h, n_strings, &grid, &p_sub);
-    if (rc) return rc;
     const int k = mode == TREX_PNFA_FP16 ? 1 : mode == TREX_PNFA_BOOL ? 2 : mode == TREX_PNFA_BOOL8 ? 3 : 0;
-    PnParams P;
-    P.data = data;
-    P.total_bytes = total_bytes;
-    P.offsets = offsets;
-    P.n = n_strings;
-    P.tpack = h->d_tpack[k];
-    P.rsym = h->d_rsym[k];
-    P.start_img = h->d_simg[k];
-    P.acc = k >= 2 ? h->d_acc_bool : h->d_acc;
-    P.start_max = h->start_max16[k];
-    P.ll_empty = k >= 2 ? h->ll_empty_bool : h->ll_empty;
-    P.boolean = k >= 2;
-    P.kcols = k == 3 ? 4 : 8;
-    P.wait_cycles = mbar_wait_cycles();
-    P.resc = k == 0 ? h->tc_resc : 1;
-    P.sigma = h->sigma;
-    P.loglik = loglik;
-    P.accept = accept;
-    P.accept_i32 = accept_i32;
-    P.queue = queue;
-    P.err = err;
-    P.L = pn_layout(p_sub, h->sigma, k == 3 ? 16 : 32);
-    // one CTA per SM: it owns all 512 TMEM columns
-    const uint32_t smem = std::max<uint32_t>(P.L.total, 120u * 1024u);
+    SyParams Q;
+    Q.data = data;
+    Q.total_bytes = total_bytes;
+    Q.offsets = offsets;
+    Q.n = n_strings;
+    Q.T16 = h->d_T16[k == 1 ? 1 : 0];
+    Q.T32 = h->d_T32;
+    Q.start_img = h->d_simg[k];
+    Q.acc = k >= 2 ? h->d_acc_bool : h->d_acc;
+    Q.sigma = h->sigma;
+    Q.rep = std::max(1, kSyWarps / h->sigma);
+    Q.rsym = h->d_rsym[k];
+    Q.start_max = h->start_max16[k];
+    Q.resc = k == 0 ? h->tc_resc : 1;
+    Q.wait_cycles = mbar_wait_cycles();
+    Q.ll_empty = k >= 2 ? h->ll_empty_bool : h->ll_empty;
+    Q.loglik = loglik;
+    Q.accept = accept;
+    Q.accept_i32 = accept_i32;
+    Q.queue = queue;
+    Q.err = err;
+    // one CTA an SM (its registers hold the tables), the strings spread over all SMs
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(n_strings, pn_sms(h)));
+    const uint32_t row = k == 3 ? sy_row_bytes<2>() : sy_row_bytes<0>();
+    uint32_t smem = 0;
+    for (Q.slots = (int)std::min<int64_t>((n_strings + grid - 1) / grid, kSyMaxSlots);; --Q.slots) {
+        const uint32_t n = (uint32_t)Q.slots;
+        Q.cap_shift = 3;
+        while ((1 << Q.cap_shift) < Q.slots) ++Q.cap_shift;
+        Q.state_off = kSyRecs + n * (uint32_t)sizeof(SyRec);
+        Q.sym_off = Q.state_off + n;
+        Q.raw_off = pn_align16(Q.sym_off + 2u * kSyBlk * n);
+        Q.list_off = Q.raw_off + 32u * n;
+        Q.rows_off = pn_align16(Q.list_off + (4u << Q.cap_shift) * (uint32_t)Q.sigma);
+        smem = Q.rows_off + n * row;
+        if (smem <= kPnSmemCap) break;
+    }
+    const int threads = 32 * std::min(kSyWarps, Q.sigma * Q.rep);
     profile_kernel_begin(st);
-    if (k == 1) pnfa_tc_kernel<1><<<grid, kPnThreads, smem, st>>>(P);
-    else if (k == 3) pnfa_tc_kernel<2><<<grid, kPnThreads, smem, st>>>(P);
-    else pnfa_tc_kernel<0><<<grid, kPnThreads, smem, st>>>(P);
+    const bool several = Q.sigma > kSyWarps;
+    void (*const f)(SyParams) = k == 1   ? (several ? pnfa_sym_kernel<1, true> : pnfa_sym_kernel<1, false>)
+                                : k == 2 ? (several ? pnfa_sym_kernel<3, true> : pnfa_sym_kernel<3, false>)
+                                : k == 3 ? (several ? pnfa_sym_kernel<2, true> : pnfa_sym_kernel<2, false>)
+                                         : (several ? pnfa_sym_kernel<0, true> : pnfa_sym_kernel<0, false>);
+    f<<<grid, threads, smem, st>>>(Q);
     profile_kernel_end(st);
     TREX_CHECK_LAUNCH();
     return TREX_OK;

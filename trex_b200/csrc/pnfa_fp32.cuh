@@ -20,19 +20,19 @@
 
 namespace trex {
 
-constexpr int kSyWarps = 20;            // 5 a scheduler: 96 registers a thread
-constexpr int kSyThreads = 32 * kSyWarps;
-constexpr int kSyMaxSlots = 512;
-constexpr uint32_t kSyNone = 0xFFFFu;
-constexpr int kSyReg = 6, kSyGroup = 4;
-constexpr uint32_t kSyTblBytes = (16 - kSyReg) * 64 * 16;   // a symbol's part in shared memory
-constexpr uint32_t kSyRowBytes = 256 + 16;   // a state row; 16 more, so that rows spread over the banks
+constexpr int kRiWarps = 20;            // 5 a scheduler: 96 registers a thread
+constexpr int kRiThreads = 32 * kRiWarps;
+constexpr int kRiMaxSlots = 512;
+constexpr uint32_t kRiNone = 0xFFFFu;
+constexpr int kRiReg = 6, kRiGroup = 4;
+constexpr uint32_t kRiTblBytes = (16 - kRiReg) * 64 * 16;   // a symbol's part in shared memory
+constexpr uint32_t kRiRowBytes = 256 + 16;   // a state row; 16 more, so that rows spread over the banks
 
 // Record of a slot's string, 32 bytes of shared memory: next byte to read, end of the string
 // (addresses), exponent sum (64 bits), string index, accept-weighted sum of an ended string.
-constexpr uint32_t kSyRecBytes = 32, kSyRecP = 0, kSyRecE = 16, kSyRecDot = 28;
+constexpr uint32_t kRiRecBytes = 32, kRiRecP = 0, kRiRecE = 16, kRiRecDot = 28;
 
-struct SyParams {
+struct RiParams {
     const uint8_t *data;
     int64_t total_bytes;
     const int64_t *offsets;
@@ -54,89 +54,89 @@ struct SyParams {
 
 // Shared memory: control words, rings (n_rings, then that of ended slots), records, state rows,
 // tables.
-constexpr uint32_t kSyTails = 0;                        // uint32 [kSyWarps + 1]
-constexpr uint32_t kSyEndHead = 128, kSyLock = 132, kSyLive = 136, kSyDone = 140;
-constexpr uint32_t kSyAcc = 144;                        // float [64]
-constexpr uint32_t kSyStart = kSyAcc + 256;             // uint4 [16]
-constexpr uint32_t kSyRings = kSyStart + 256;           // uint16 [n_rings + 1][ring_cap]
+constexpr uint32_t kRiTails = 0;                        // uint32 [kRiWarps + 1]
+constexpr uint32_t kRiEndHead = 128, kRiLock = 132, kRiLive = 136, kRiDone = 140;
+constexpr uint32_t kRiAcc = 144;                        // float [64]
+constexpr uint32_t kRiStart = kRiAcc + 256;             // uint4 [16]
+constexpr uint32_t kRiRings = kRiStart + 256;           // uint16 [n_rings + 1][ring_cap]
 
 // ---- 32-bit shared addresses (a generic pointer would take two registers)
-extern __shared__ __align__(16) uint8_t sy_smem[];
-__device__ __forceinline__ uint32_t sy_base() { return pn_smem_u32(sy_smem); }
-__device__ __forceinline__ uint32_t sy_ld32(uint32_t a) {
+extern __shared__ __align__(16) uint8_t ri_smem[];
+__device__ __forceinline__ uint32_t ri_base() { return pn_smem_u32(ri_smem); }
+__device__ __forceinline__ uint32_t ri_ld32(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t sy_ld16(uint32_t a) {
+__device__ __forceinline__ uint32_t ri_ld16(uint32_t a) {
     uint16_t v;
     asm volatile("ld.volatile.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ uint2 sy_ld64(uint32_t a) {
+__device__ __forceinline__ uint2 ri_ld64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ uint4 sy_ld128(uint32_t a) {
+__device__ __forceinline__ uint4 ri_ld128(uint32_t a) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ void sy_ldp(uint32_t a, const uint8_t *&p, const uint8_t *&e) {
+__device__ __forceinline__ void ri_ldp(uint32_t a, const uint8_t *&p, const uint8_t *&e) {
     asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(p), "=l"(e) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void sy_stp(uint32_t a, const uint8_t *p) {
+__device__ __forceinline__ void ri_stp(uint32_t a, const uint8_t *p) {
     asm volatile("st.shared.u64 [%0], %1;" :: "r"(a), "l"(p) : "memory");
 }
-__device__ __forceinline__ void sy_st16(uint32_t a, uint32_t v) {
+__device__ __forceinline__ void ri_st16(uint32_t a, uint32_t v) {
     asm volatile("st.volatile.shared.u16 [%0], %1;" :: "r"(a), "h"((uint16_t)v) : "memory");
 }
-__device__ __forceinline__ void sy_st32(uint32_t a, uint32_t v) {
+__device__ __forceinline__ void ri_st32(uint32_t a, uint32_t v) {
     asm volatile("st.volatile.shared.u32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
 }
-__device__ __forceinline__ void sy_st64(uint32_t a, uint32_t x, uint32_t y) {
+__device__ __forceinline__ void ri_st64(uint32_t a, uint32_t x, uint32_t y) {
     asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(a), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void sy_st128(uint32_t a, uint4 v) {
+__device__ __forceinline__ void ri_st128(uint32_t a, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ uint32_t sy_add32(uint32_t a, uint32_t v) {
+__device__ __forceinline__ uint32_t ri_add32(uint32_t a, uint32_t v) {
     uint32_t o;
     asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
     return o;
 }
-__device__ __forceinline__ void sy_fence() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+__device__ __forceinline__ void ri_fence() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
 // Address of entry `pos` of ring `ring`.
-__device__ __forceinline__ uint32_t sy_entry(const SyParams &P, uint32_t ring, uint32_t pos) {
-    return sy_base() + kSyRings + 2u * (ring * (uint32_t)P.ring_cap + (pos & (uint32_t)(P.ring_cap - 1)));
+__device__ __forceinline__ uint32_t ri_entry(const RiParams &P, uint32_t ring, uint32_t pos) {
+    return ri_base() + kRiRings + 2u * (ring * (uint32_t)P.ring_cap + (pos & (uint32_t)(P.ring_cap - 1)));
 }
 // The ring in which slot waits for symbol c.
-__device__ __forceinline__ uint32_t sy_ring_of(const SyParams &P, uint32_t c, uint32_t slot) {
+__device__ __forceinline__ uint32_t ri_ring_of(const RiParams &P, uint32_t c, uint32_t slot) {
     return c + (uint32_t)P.sigma * ((slot * (uint32_t)P.rep) >> P.rep_shift);
 }
 // Puts a slot in a ring, after its row and record were written (by this thread, or by its warp
 // before a __syncwarp): the fence makes them visible to the warp that finds the entry. A ring
 // holds as many entries as there are slots and a slot is in one ring at a time, so an entry is
 // read before its place is used again.
-__device__ __forceinline__ void sy_push(const SyParams &P, uint32_t ring, uint32_t slot) {
-    sy_fence();
-    const uint32_t pos = sy_add32(sy_base() + kSyTails + 4u * ring, 1u);
-    sy_st16(sy_entry(P, ring, pos), slot);
+__device__ __forceinline__ void ri_push(const RiParams &P, uint32_t ring, uint32_t slot) {
+    ri_fence();
+    const uint32_t pos = ri_add32(ri_base() + kRiTails + 4u * ring, 1u);
+    ri_st16(ri_entry(P, ring, pos), slot);
 }
 // The entries at the front of a ring: this lane's entry (lanes below `most`); returns how many.
-__device__ __forceinline__ uint32_t sy_poll(const SyParams &P, uint32_t ring, uint32_t head, uint32_t most,
+__device__ __forceinline__ uint32_t ri_poll(const RiParams &P, uint32_t ring, uint32_t head, uint32_t most,
                                             uint32_t &ent) {
     const uint32_t lane = threadIdx.x & 31u;
-    ent = kSyNone;
-    if (lane < most) ent = sy_ld16(sy_entry(P, ring, head + lane));
-    const uint32_t got = __ballot_sync(0xffffffffu, ent != kSyNone);
+    ent = kRiNone;
+    if (lane < most) ent = ri_ld16(ri_entry(P, ring, head + lane));
+    const uint32_t got = __ballot_sync(0xffffffffu, ent != kRiNone);
     return got == 0xffffffffu ? 32u : (uint32_t)__ffs(~got) - 1u;
 }
 
 // Gives a slot the next string of the batch: its record, its start row and its first ring.
 // Strings without symbols get their result at once; false when the batch has no more strings.
-__device__ __forceinline__ bool sy_refill(const SyParams &P, uint32_t slot) {
+__device__ __forceinline__ bool ri_refill(const RiParams &P, uint32_t slot) {
     for (;;) {
         const unsigned long long idx = atomicAdd(P.queue, 1ull);
         if (idx >= (unsigned long long)P.n) return false;
@@ -152,63 +152,63 @@ __device__ __forceinline__ bool sy_refill(const SyParams &P, uint32_t slot) {
             pn_write_result(P.loglik, P.accept, P.accept_i32, (int64_t)idx, P.ll_empty);
             continue;
         }
-        const uint32_t rec = sy_base() + P.recs_off + slot * kSyRecBytes;
-        sy_stp(rec + kSyRecP, p + 1);
-        sy_stp(rec + kSyRecP + 8u, e);
-        sy_st128(rec + kSyRecE, make_uint4(0u, 0u, (uint32_t)idx, 0u));
-        const uint32_t row = sy_base() + P.rows_off + slot * kSyRowBytes;
-        for (uint32_t k = 0; k < kSyRowBytes - 16u; k += 16u) sy_st128(row + k, sy_ld128(sy_base() + kSyStart + k));
-        sy_push(P, sy_ring_of(P, c, slot), slot);
+        const uint32_t rec = ri_base() + P.recs_off + slot * kRiRecBytes;
+        ri_stp(rec + kRiRecP, p + 1);
+        ri_stp(rec + kRiRecP + 8u, e);
+        ri_st128(rec + kRiRecE, make_uint4(0u, 0u, (uint32_t)idx, 0u));
+        const uint32_t row = ri_base() + P.rows_off + slot * kRiRowBytes;
+        for (uint32_t k = 0; k < kRiRowBytes - 16u; k += 16u) ri_st128(row + k, ri_ld128(ri_base() + kRiStart + k));
+        ri_push(P, ri_ring_of(P, c, slot), slot);
         return true;
     }
 }
 
 // The ended slots, up to 32 at a time (the calling warp holds the lock): results, next strings.
 // The last slot without a string ends the kernel's work.
-__device__ __noinline__ void sy_feed(const SyParams &P) {
+__device__ __noinline__ void ri_feed(const RiParams &P) {
     const uint32_t FULL = 0xffffffffu, lane = threadIdx.x & 31u;
-    const uint32_t head = sy_ld32(sy_base() + kSyEndHead);
+    const uint32_t head = ri_ld32(ri_base() + kRiEndHead);
     uint32_t slot;
-    const uint32_t cnt = sy_poll(P, (uint32_t)P.n_rings, head, 32u, slot);
+    const uint32_t cnt = ri_poll(P, (uint32_t)P.n_rings, head, 32u, slot);
     bool retired = false;
     if (lane < cnt) {
-        sy_fence();
-        sy_st16(sy_entry(P, (uint32_t)P.n_rings, head + lane), kSyNone);
-        const uint4 w = sy_ld128(sy_base() + P.recs_off + slot * kSyRecBytes + kSyRecE);
+        ri_fence();
+        ri_st16(ri_entry(P, (uint32_t)P.n_rings, head + lane), kRiNone);
+        const uint4 w = ri_ld128(ri_base() + P.recs_off + slot * kRiRecBytes + kRiRecE);
         const double dot = (double)__uint_as_float(w.w);
         const int64_t E = (int64_t)(((uint64_t)w.y << 32) | w.x);
         pn_write_result(P.loglik, P.accept, P.accept_i32, (int64_t)w.z,
                         dot > 0.0 ? log(dot) + (double)E * 0.69314718055994530942 : -INFINITY);
-        retired = !sy_refill(P, slot);
+        retired = !ri_refill(P, slot);
     }
     const uint32_t gone = (uint32_t)__popc(__ballot_sync(FULL, retired));
     if (lane == 0) {
-        sy_st32(sy_base() + kSyEndHead, head + cnt);
-        if (gone && sy_add32(sy_base() + kSyLive, 0u - gone) == gone) sy_st32(sy_base() + kSyDone, 1u);
-        sy_fence();
-        sy_st32(sy_base() + kSyLock, 0u);
+        ri_st32(ri_base() + kRiEndHead, head + cnt);
+        if (gone && ri_add32(ri_base() + kRiLive, 0u - gone) == gone) ri_st32(ri_base() + kRiDone, 1u);
+        ri_fence();
+        ri_st32(ri_base() + kRiLock, 0u);
     }
     __syncwarp();
 }
 // Feeds when slots are waiting (at least `least`) and no other warp does.
-__device__ __forceinline__ bool sy_try_feed(const SyParams &P, uint32_t least) {
-    const uint32_t tail = sy_ld32(sy_base() + kSyTails + 4u * (uint32_t)P.n_rings);
-    if (tail - sy_ld32(sy_base() + kSyEndHead) < least) return false;
+__device__ __forceinline__ bool ri_try_feed(const RiParams &P, uint32_t least) {
+    const uint32_t tail = ri_ld32(ri_base() + kRiTails + 4u * (uint32_t)P.n_rings);
+    if (tail - ri_ld32(ri_base() + kRiEndHead) < least) return false;
     uint32_t got = 0u;
     if ((threadIdx.x & 31u) == 0u)
-        asm volatile("atom.shared.cas.b32 %0, [%1], 0, 1;" : "=r"(got) : "r"(sy_base() + kSyLock) : "memory");
+        asm volatile("atom.shared.cas.b32 %0, [%1], 0, 1;" : "=r"(got) : "r"(ri_base() + kRiLock) : "memory");
     if (__shfl_sync(0xffffffffu, got, 0) != 0u) return false;
-    sy_fence();
-    sy_feed(P);
+    ri_fence();
+    ri_feed(P);
     return true;
 }
 
 // A wait without work: true when nothing moved in any ring for `limit` clock cycles (all lanes
 // call it; mark and t0 carry over between calls).
-__device__ __forceinline__ bool sy_stalled(const SyParams &P, uint32_t &mark, long long &t0) {
+__device__ __forceinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
     const uint32_t lane = threadIdx.x & 31u;
     if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) return false;
-    const uint32_t v = (int)lane <= P.n_rings ? sy_ld32(sy_base() + kSyTails + 4u * lane) : 0u;
+    const uint32_t v = (int)lane <= P.n_rings ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
     const uint32_t sum = __reduce_add_sync(0xffffffffu, v);
     if (sum == mark) return true;
     mark = sum;
@@ -218,18 +218,18 @@ __device__ __forceinline__ bool sy_stalled(const SyParams &P, uint32_t &mark, lo
 
 // Waits for entries of a ring (up to `most`), feeding ended slots meanwhile; 0 when the work is
 // done (or the wait gave up).
-__device__ __forceinline__ uint32_t sy_wait(const SyParams &P, uint32_t ring, uint32_t head, uint32_t most, uint32_t &ent) {
+__device__ __forceinline__ uint32_t ri_wait(const RiParams &P, uint32_t ring, uint32_t head, uint32_t most, uint32_t &ent) {
     uint32_t cnt, mark = 0u;
     long long t0 = 0;
-    sy_try_feed(P, 32u);
-    while ((cnt = sy_poll(P, ring, head, most, ent)) == 0u) {
-        if (sy_ld32(sy_base() + kSyDone)) return 0u;
-        if (sy_try_feed(P, 1u)) continue;
+    ri_try_feed(P, 32u);
+    while ((cnt = ri_poll(P, ring, head, most, ent)) == 0u) {
+        if (ri_ld32(ri_base() + kRiDone)) return 0u;
+        if (ri_try_feed(P, 1u)) continue;
         if (t0 == 0) t0 = clock64();
-        if (sy_stalled(P, mark, t0)) {
+        if (ri_stalled(P, mark, t0)) {
             if ((threadIdx.x & 31u) == 0u) {
                 atomicOr(P.err, kPnErrTimeout);
-                sy_st32(sy_base() + kSyDone, 1u);
+                ri_st32(ri_base() + kRiDone, 1u);
             }
             return 0u;
         }
@@ -238,42 +238,42 @@ __device__ __forceinline__ uint32_t sy_wait(const SyParams &P, uint32_t ring, ui
 }
 
 // Clears the control words, copies the small tables in and gives every slot its first string.
-__device__ __forceinline__ void sy_init(const SyParams &P) {
-    uint32_t *w = reinterpret_cast<uint32_t *>(sy_smem);
-    for (uint32_t i = threadIdx.x; i < kSyAcc / 4; i += blockDim.x) w[i] = 0u;
-    for (int i = threadIdx.x; i < (P.n_rings + 1) * P.ring_cap / 2; i += blockDim.x) w[kSyRings / 4 + i] = 0xFFFFFFFFu;
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) reinterpret_cast<float *>(sy_smem + kSyAcc)[i] = P.acc[i];
-    if (threadIdx.x < 16) reinterpret_cast<uint4 *>(sy_smem + kSyStart)[threadIdx.x] = P.start_img[threadIdx.x];
+__device__ __forceinline__ void ri_init(const RiParams &P) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(ri_smem);
+    for (uint32_t i = threadIdx.x; i < kRiAcc / 4; i += blockDim.x) w[i] = 0u;
+    for (int i = threadIdx.x; i < (P.n_rings + 1) * P.ring_cap / 2; i += blockDim.x) w[kRiRings / 4 + i] = 0xFFFFFFFFu;
+    for (int i = threadIdx.x; i < 64; i += blockDim.x) reinterpret_cast<float *>(ri_smem + kRiAcc)[i] = P.acc[i];
+    if (threadIdx.x < 16) reinterpret_cast<uint4 *>(ri_smem + kRiStart)[threadIdx.x] = P.start_img[threadIdx.x];
     __syncthreads();
-    if (threadIdx.x == 0) w[kSyLive / 4] = (uint32_t)P.slots;
+    if (threadIdx.x == 0) w[kRiLive / 4] = (uint32_t)P.slots;
     __syncthreads();
     for (uint32_t slot = threadIdx.x; slot < (uint32_t)P.slots; slot += blockDim.x)
-        if (!sy_refill(P, slot) && sy_add32(sy_base() + kSyLive, 0xffffffffu) == 1u) sy_st32(sy_base() + kSyDone, 1u);
+        if (!ri_refill(P, slot) && ri_add32(ri_base() + kRiLive, 0xffffffffu) == 1u) ri_st32(ri_base() + kRiDone, 1u);
     __syncwarp();
 }
 
 // One group's products: row `lane` and row `lane` + 32 of the table times the states of G strings.
 template <int G>
-__device__ __forceinline__ void sy_products(const float4 (&t)[2][kSyReg], uint32_t tbl, const uint32_t (&row)[kSyGroup],
-                                              float (&a)[kSyGroup][2]) {
+__device__ __forceinline__ void ri_products(const float4 (&t)[2][kRiReg], uint32_t tbl, const uint32_t (&row)[kRiGroup],
+                                              float (&a)[kRiGroup][2]) {
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
     for (int g = 0; g < G; ++g) a[g][0] = a[g][1] = 0.f;
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         float4 t0, t1;
-        if (k < kSyReg) {
-            t0 = t[0][k < kSyReg ? k : 0];
-            t1 = t[1][k < kSyReg ? k : 0];
+        if (k < kRiReg) {
+            t0 = t[0][k < kRiReg ? k : 0];
+            t1 = t[1][k < kRiReg ? k : 0];
         } else {
-            const uint32_t at = tbl + (uint32_t)(k - kSyReg) * 1024u + lane * 16u;
-            const uint4 u = sy_ld128(at), v = sy_ld128(at + 512u);
+            const uint32_t at = tbl + (uint32_t)(k - kRiReg) * 1024u + lane * 16u;
+            const uint4 u = ri_ld128(at), v = ri_ld128(at + 512u);
             t0 = make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
             t1 = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
         }
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            const uint4 x = sy_ld128(row[g] + 16u * k);
+            const uint4 x = ri_ld128(row[g] + 16u * k);
             a[g][0] = fmaf(t0.x, __uint_as_float(x.x), a[g][0]);
             a[g][0] = fmaf(t0.y, __uint_as_float(x.y), a[g][0]);
             a[g][0] = fmaf(t0.z, __uint_as_float(x.z), a[g][0]);
@@ -286,53 +286,53 @@ __device__ __forceinline__ void sy_products(const float4 (&t)[2][kSyReg], uint32
     }
 }
 
-__global__ void __launch_bounds__(kSyThreads, 1) pnfa_fp32_kernel(const __grid_constant__ SyParams P) {
+__global__ void __launch_bounds__(kRiThreads, 1) pnfa_fp32_kernel(const __grid_constant__ RiParams P) {
     const uint32_t FULL = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     // pieces 6 .. 15 of every table: [symbol][piece][row] float4
-    for (int i = threadIdx.x; i < P.sigma * (16 - kSyReg) * 64; i += blockDim.x) {
-        const int c = i / ((16 - kSyReg) * 64), rest = i % ((16 - kSyReg) * 64);
-        const int k = kSyReg + rest / 64, r = rest % 64;
-        *reinterpret_cast<float4 *>(sy_smem + P.tbl_off + 16 * (size_t)i) =
+    for (int i = threadIdx.x; i < P.sigma * (16 - kRiReg) * 64; i += blockDim.x) {
+        const int c = i / ((16 - kRiReg) * 64), rest = i % ((16 - kRiReg) * 64);
+        const int k = kRiReg + rest / 64, r = rest % 64;
+        *reinterpret_cast<float4 *>(ri_smem + P.tbl_off + 16 * (size_t)i) =
             __ldg(reinterpret_cast<const float4 *>(P.T32 + ((size_t)c * 64 + r) * 64) + k);
     }
     const uint32_t ring = warp, c = ring % (uint32_t)P.sigma;
-    float4 t[2][kSyReg];
+    float4 t[2][kRiReg];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int k = 0; k < kSyReg; ++k)
+        for (int k = 0; k < kRiReg; ++k)
             t[h][k] = __ldg(reinterpret_cast<const float4 *>(P.T32 + ((size_t)c * 64 + 32 * h + lane) * 64) + k);
-    sy_init(P);   // (its barriers also cover the tables)
-    const uint32_t tbl = sy_base() + P.tbl_off + c * kSyTblBytes;
+    ri_init(P);   // (its barriers also cover the tables)
+    const uint32_t tbl = ri_base() + P.tbl_off + c * kRiTblBytes;
     uint32_t head = 0u;
     for (;;) {
         uint32_t ent;
-        const uint32_t cnt = sy_wait(P, ring, head, kSyGroup, ent);
+        const uint32_t cnt = ri_wait(P, ring, head, kRiGroup, ent);
         if (cnt == 0u) return;
-        sy_fence();
-        if (lane < cnt) sy_st16(sy_entry(P, ring, head + lane), kSyNone);
+        ri_fence();
+        if (lane < cnt) ri_st16(ri_entry(P, ring, head + lane), kRiNone);
         head += cnt;
         const bool own = lane < cnt;   // lanes 0 .. cnt - 1 keep the records
-        const uint32_t rec = sy_base() + P.recs_off + (own ? ent : 0u) * kSyRecBytes;
+        const uint32_t rec = ri_base() + P.recs_off + (own ? ent : 0u) * kRiRecBytes;
         uint32_t nc = 255u;
         if (own) {
             const uint8_t *p, *e;
-            sy_ldp(rec + kSyRecP, p, e);
+            ri_ldp(rec + kRiRecP, p, e);
             if (p < e) nc = __ldg(p);
         }
-        uint32_t row[kSyGroup];
+        uint32_t row[kRiGroup];
 #pragma unroll
-        for (int g = 0; g < kSyGroup; ++g)
-            row[g] = sy_base() + P.rows_off + __shfl_sync(FULL, ent, g < (int)cnt ? g : 0) * kSyRowBytes;
-        float a[kSyGroup][2];
-        if (cnt == 1u) sy_products<1>(t, tbl, row, a);
-        else if (cnt == 2u) sy_products<2>(t, tbl, row, a);
-        else sy_products<4>(t, tbl, row, a);
+        for (int g = 0; g < kRiGroup; ++g)
+            row[g] = ri_base() + P.rows_off + __shfl_sync(FULL, ent, g < (int)cnt ? g : 0) * kRiRowBytes;
+        float a[kRiGroup][2];
+        if (cnt == 1u) ri_products<1>(t, tbl, row, a);
+        else if (cnt == 2u) ri_products<2>(t, tbl, row, a);
+        else ri_products<4>(t, tbl, row, a);
         bool ending = false;
         if (own) {   // the symbol after this one (bytes >= sigma are skipped)
             const uint8_t *p, *e;
-            sy_ldp(rec + kSyRecP, p, e);
+            ri_ldp(rec + kRiRecP, p, e);
             bool found = p < e && nc < (uint32_t)P.sigma;
             if (p < e) ++p;
             while (!found && p < e) {
@@ -340,11 +340,11 @@ __global__ void __launch_bounds__(kSyThreads, 1) pnfa_fp32_kernel(const __grid_c
                 found = nc < (uint32_t)P.sigma;
             }
             ending = !found;
-            sy_stp(rec + kSyRecP, p);
+            ri_stp(rec + kRiRecP, p);
         }
         const uint32_t ends = __ballot_sync(FULL, ending);
 #pragma unroll
-        for (int g = 0; g < kSyGroup; ++g) {
+        for (int g = 0; g < kRiGroup; ++g) {
             if (g >= (int)cnt) break;
             // frexp exponent of max|s'|, then the exact scale (NaN as the plain kernel's fmaxf: ignored)
             const uint32_t mb = __reduce_max_sync(
@@ -369,25 +369,25 @@ __global__ void __launch_bounds__(kSyThreads, 1) pnfa_fp32_kernel(const __grid_c
                     s1 *= sc2;
                 }
                 if ((int)lane == g) {
-                    const uint2 w = sy_ld64(rec + kSyRecE);
+                    const uint2 w = ri_ld64(rec + kRiRecE);
                     const int64_t E = (int64_t)(((uint64_t)w.y << 32) | w.x) + e;
-                    sy_st64(rec + kSyRecE, (uint32_t)E, (uint32_t)((uint64_t)E >> 32));
+                    ri_st64(rec + kRiRecE, (uint32_t)E, (uint32_t)((uint64_t)E >> 32));
                 }
             }
             __syncwarp();   // every lane has read the row
             if ((ends >> g) & 1u) {
-                float d = s0 * __uint_as_float(sy_ld32(sy_base() + kSyAcc + 4u * lane)) +
-                          s1 * __uint_as_float(sy_ld32(sy_base() + kSyAcc + 4u * lane + 128u));
+                float d = s0 * __uint_as_float(ri_ld32(ri_base() + kRiAcc + 4u * lane)) +
+                          s1 * __uint_as_float(ri_ld32(ri_base() + kRiAcc + 4u * lane + 128u));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(FULL, d, o);
-                if ((int)lane == g) sy_st32(rec + kSyRecDot, __float_as_uint(d));
+                if ((int)lane == g) ri_st32(rec + kRiRecDot, __float_as_uint(d));
             } else {
-                sy_st32(row[g] + 4u * lane, __float_as_uint(s0));
-                sy_st32(row[g] + 4u * lane + 128u, __float_as_uint(s1));
+                ri_st32(row[g] + 4u * lane, __float_as_uint(s0));
+                ri_st32(row[g] + 4u * lane + 128u, __float_as_uint(s1));
             }
         }
         __syncwarp();
-        if (own) sy_push(P, ending ? (uint32_t)P.n_rings : sy_ring_of(P, nc, ent), ent);
+        if (own) ri_push(P, ending ? (uint32_t)P.n_rings : ri_ring_of(P, nc, ent), ent);
         __syncwarp();
     }
 }

@@ -306,15 +306,15 @@ class PNFA:
     result log(dot(s_L, accept)) in FP64 (reference
     cuda/nfa_tc_evolution.cu:456-610 computes only dot > 0.5).
 
-    Modes: "bf16" / "fp16" run the tcgen05 tensor-core kernel (16-bit
+    Modes: "bf16" / "fp16" run the tensor-core kernels (16-bit
     operands, FP32 accumulation, sigma <= 28); "fp32" the CUDA-core kernel.
     "bool" runs the Boolean NFA of the same tables on the tensor cores (the
     reference's FP16 WMMA nfa_tc_binary kernels, cuda/nfa_tc_evolution.cu:
     59-442): nonzero entries are edges, each product is thresholded to {0, 1}
     (exact), accept = some accepting state active; loglik is then the log of
     the number of active accepting states. Bytes >= sigma are skipped.
-    "bool8": the same Boolean NFA with 0/1 int8 operands and int32 sums (tcgen05
-    kind::i8, K = 32 an instruction: half the MMA instructions of "bool").
+    "bool8": the same Boolean NFA with 0/1 int8 operands and int32 sums (K = 32 an
+    MMA instruction: half the instructions of "bool").
     "bf16cc" / "fp16cc": CUDA cores with the 16-bit tables in shared memory and an
     FP32 state, four warps per string: the low-latency form for few strings.
     """

@@ -367,7 +367,7 @@ class Server:
                 m.set_sm_limit(max(1, pnfa_sms // max(1, min(kAuxStreams, pnfa_streams))))
         # "auto": the CUDA-core kernel with BF16 tables in shared memory for groups of fewer
         # than pnfa_auto_threshold strings (its per-step latency is far lower than the
-        # tensor-core kernel's), BF16 tcgen05 above
+        # tensor-core kernel's), BF16 tensor cores above
         if pnfa_mode not in ("bf16", "fp16", "fp32", "bf16cc", "fp16cc", "auto"):
             raise ValueError("pnfa_mode must be bf16, fp16, fp32, bf16cc, fp16cc or auto")
         self.pnfa_mode = pnfa_mode
