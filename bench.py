@@ -1172,7 +1172,7 @@ def measure(wl, args, torch, dev, *, steps, warmup, rank=0, world=1, local_rank=
                 "frac": achieved / peak, "traffic": traffic, "kernel": wl.kernel,
                 "kernel_ms_mean": kmean, "algorithmic_flops_per_launch": wl.alg_flops,
                 "peak_source": f"MEASURED_PEAKS.json bf16_tflops_sustained ({peak_kind}); "
-                               "useful flops 2*64*64 per symbol (the pair layout issues 2x)"}
+                               "useful flops 2*64*64 per symbol"}
     else:
         peak, peak_kind = measured_peaks()
         achieved = wl.alg_bytes / (kmean * 1e-3) / 1e9

@@ -66,32 +66,22 @@ __device__ __forceinline__ bool pn_mbar_test(uint32_t addr, uint32_t parity) {
         : "=r"(done) : "r"(addr), "r"(parity) : "memory");
     return done != 0;
 }
-__device__ __forceinline__ void pn_mbar_arrive(uint32_t addr) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(addr) : "memory");
-}
-
-// Waits (lane 0 of the calling warp) for the completion of the phase with the given parity;
-// bounded; the result is broadcast to the warp. A thread whose phase is not complete may be
-// parked by the hardware (try_wait) instead of spinning, which leaves the issue slots to the
-// warps with work.
-__device__ __forceinline__ bool pn_wait_park(uint32_t addr, uint32_t parity, volatile uint32_t *abort_flag,
-                                             uint32_t *err, long long limit) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) {
-        const long long t0 = clock64();
-        while (!pn_mbar_test(addr, parity)) {
-            if (*abort_flag) { ok = 0; break; }
-            if (clock64() - t0 > limit) {
-                atomicOr(err, kPnErrTimeout);
-                *abort_flag = 1u;
-                ok = 0;
-                break;
-            }
+// The warp waits for the completion of the phase with the given parity; bounded, the same result
+// in all lanes. A thread whose phase is not complete may be parked by the hardware (try_wait).
+__device__ __forceinline__ bool ln_wait(uint32_t addr, uint32_t parity, volatile uint32_t *abort_flag,
+                                        uint32_t *err, long long limit) {
+    bool ok = true;
+    const long long t0 = clock64();
+    while (!pn_mbar_test(addr, parity)) {
+        if (*abort_flag) { ok = false; break; }
+        if (clock64() - t0 > limit) {
+            atomicOr(err, kPnErrTimeout);
+            *abort_flag = 1u;
+            ok = false;
+            break;
         }
     }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
+    return __all_sync(0xffffffffu, ok);
 }
 
 __device__ __forceinline__ void pn_write_result(double *loglik, uint8_t *accept, int32_t *accept_i32,
@@ -149,15 +139,20 @@ __device__ __forceinline__ void pn_tmem_st16(uint32_t taddr, const uint32_t (&r)
 // The epilogue is thread-local (thread = TMEM lane = string): it reads its 64 states, finds
 // their maximum and rescales by an exact power of two, rounds them to the operand type and
 // writes its next A row with tcgen05.st; at the string's end it forms the log-likelihood and
-// takes the next string from the queue. The MMA warp issues the tiles round robin, so the
-// epilogue of one tile overlaps the products of the others. Hand-offs per tile: `full`
-// (tcgen05.commit, one arrival) and `ready` (the four epilogue warps, after their A rows and a
-// liveness flag are written); every wait is bounded.
+// takes the next string from the queue.
+//
+// Bound by the latency of a tile's step (the 512 TMEM columns hold no more strings): 4900 cycles
+// before, alike with one tile and with four, now about half. 262144 strings x 2048 symbols, 2 symbols,
+// FP16: 20.27 -> 10.70 ms; x 512 symbols, ms before / now, for 2, 3, 4 symbols: BF16 4.58 / 2.46,
+// 5.88 / 3.12, 8.37 / 4.26; FP16 5.14 / 2.85, 6.49 / 3.41, 9.14 / 4.65; int8 4.87 / 2.15, 4.98 / 2.29,
+// 5.15 / 2.53. Before, warps of their own waited at an mbarrier for the tile, read its liveness
+// from shared memory and issued the products, and the next symbol was found after them.
+// So a step has one hand-off: the four warps of a tile meet at a hardware barrier, which also
+// tells whether any string is left, an elected thread of the first issues the products, and the
+// next symbol is found while they run; a tcgen05.commit brings the result (a bounded wait).
 constexpr int kLnTiles = 4;
 constexpr int kLnEpiWarps = 4 * kLnTiles;   // tile T: warps 4T .. 4T + 3 (lane quadrants 0-3)
-constexpr int kLnMmaWarp = kLnEpiWarps;
-constexpr int kLnMmaWarps = 2;         // issuers: warp kLnMmaWarp + i takes tiles i, i + 2
-constexpr int kLnThreads = 32 * (kLnEpiWarps + kLnMmaWarps);
+constexpr int kLnThreads = 32 * kLnEpiWarps;
 constexpr int kLnMaxSigma = 4;
 constexpr uint32_t kLnLbo = 1024;           // B: bytes between 16-byte K columns (64 rows x 16 B)
 
@@ -241,11 +236,35 @@ __device__ __noinline__ void ln_finish(const LnParams &P, int64_t seq, float dot
     pn_write_result(P.loglik, P.accept, P.accept_i32, seq, ll);
 }
 
-__device__ __forceinline__ void ln_tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-                    "r"(r[7])
-                 : "memory");
+// Waits for this thread's TMEM loads; r is named so that nothing reads it before.
+__device__ __forceinline__ void ln_tmem_wait32(uint32_t *r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                 "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                 "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                 "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :: "memory");
+}
+// The 128 threads of tile T meet; whether any of them passed true.
+__device__ __forceinline__ bool ln_tile_any(int T, bool v) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+        "barrier.cta.red.or.pred p, %1, 128, q;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(any) : "r"(T + 1), "r"((uint32_t)v) : "memory");
+    return any != 0u;
+}
+__device__ __forceinline__ bool ln_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0u;
+}
+// max(a, |b|, |c|), a >= 0 (a NaN is passed over)
+__device__ __forceinline__ float ln_max_abs3(float a, float b, float c) {
+    float m;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
 }
 
 __device__ __forceinline__ void ln_tmem_ld32(uint32_t taddr, uint32_t *r) {
@@ -264,16 +283,12 @@ __device__ __forceinline__ void ln_tmem_ld32(uint32_t taddr, uint32_t *r) {
 // 2 = Boolean 0/1 int8 (kind::i8, int32 sums); 3 = Boolean 0/1 BF16. The Boolean forms
 // threshold every product to {0, 1} (exact).
 template <int KIND>
-__global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(LnParams P) {
+__global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(const __grid_constant__ LnParams P) {
     constexpr bool I8 = KIND == 2, BOOL = KIND >= 2, FP16 = KIND == 1;
     __shared__ __align__(1024) uint8_t s_b[64 * 64 * kLnMaxSigma * 2];
-    __shared__ __align__(8) uint64_t s_bar[2 * kLnTiles];   // full[T], then ready[T]
+    __shared__ __align__(8) uint64_t s_bar[kLnTiles];   // a tile's products are complete
     __shared__ uint32_t s_tmem, s_abort;
-    // liveness flags of a tile's four warps per ready phase parity (a warp can write the next
-    // phase's flag while another still reads this phase's)
-    __shared__ uint32_t s_alive[kLnTiles][2][4];
     __shared__ float s_acc[64], s_start[64];
-    __shared__ uint32_t s_start8[16];   // int8 Boolean form: the start set, four states a word
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sig = P.sigma;
     const int K = 64 * sig;
@@ -315,20 +330,14 @@ __global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(LnParams P) {
         s_acc[threadIdx.x] = P.acc[threadIdx.x];
         s_start[threadIdx.x] = P.start[threadIdx.x];
     }
-    if (threadIdx.x < 16) {
-        uint32_t w = 0u;
-        for (int b = 0; b < 4; ++b) w |= (P.start[4 * threadIdx.x + b] != 0.f ? 1u : 0u) << (8 * b);
-        s_start8[threadIdx.x] = w;
-    }
     if (threadIdx.x == 0) {
         s_abort = 0u;
-        for (int T = 0; T < kLnTiles; ++T) {
+        for (int T = 0; T < kLnTiles; ++T)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(pn_smem_u32(&s_bar[T])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" :: "r"(pn_smem_u32(&s_bar[kLnTiles + T])));
-        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kLnMmaWarp) {
+    __syncwarp();
+    if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(pn_smem_u32(&s_tmem)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -339,11 +348,19 @@ __global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(LnParams P) {
     pn_tc_after();
     const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(&s_tmem);
     volatile uint32_t *abort_flag = &s_abort;
-    if (warp < kLnEpiWarps && (warp >> 2) < P.tiles) {   // fewer tiles for larger alphabets
-        const int T = warp >> 2, qd = warp & 3;
-        const uint32_t tA = tbase + ((uint32_t)(32 * qd) << 16) + (uint32_t)T * P.tile_cols;
-        const uint32_t tD = tA + P.a_cols;
-        const uint32_t bar_full = pn_smem_u32(&s_bar[T]), bar_ready = pn_smem_u32(&s_bar[kLnTiles + T]);
+    if ((warp >> 2) < P.tiles) {   // fewer tiles for larger alphabets
+        // (broadcast, so that the operands of the MMAs are known to be the same in all lanes)
+        const int T = __shfl_sync(0xffffffffu, warp >> 2, 0), qd = __shfl_sync(0xffffffffu, warp & 3, 0);
+        const uint32_t tile = __shfl_sync(0xffffffffu, tbase, 0) + (uint32_t)T * P.tile_cols;
+        const uint32_t tA = tile + ((uint32_t)(32 * qd) << 16), tD = tA + P.a_cols;
+        const uint32_t bar_full = pn_smem_u32(&s_bar[T]);
+        const uint32_t fmt = KIND == 1 ? 0u : 1u;
+        const uint32_t idesc = I8 ? ((2u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24))
+                                  : ((1u << 4) | (fmt << 7) | (fmt << 10) | ((64u >> 3) << 17) |
+                                     ((128u >> 4) << 24));
+        const uint32_t sb = pn_smem_u32(s_b);
+        const uint64_t desc0 = (uint64_t)(((sb >> 4) & 0x3FFFu) | ((kLnLbo >> 4) << 16)) |
+                               ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
         const uintptr_t lo = reinterpret_cast<uintptr_t>(P.data), hi = lo + (uintptr_t)P.total_bytes;
         LnSym sy{0, 0, 0, 0, 0};
         int64_t seq = -1;
@@ -366,68 +383,105 @@ __global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(LnParams P) {
             }
         };
         bool live = fetch();
-        // A row chunk j (states 32 j .. 32 j + 31) of this string: in the K range of symbol c, zeros
-        // in the other ranges (tcgen05.st is warp-wide; each thread supplies its own row)
-        auto store_chunk = [&](int j, const float (&v)[32]) {
-            if constexpr (I8) {
-                uint32_t r[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    r[k] = (v[4 * k] != 0.f ? 1u : 0u) | (v[4 * k + 1] != 0.f ? 0x100u : 0u) |
-                           (v[4 * k + 2] != 0.f ? 0x10000u : 0u) | (v[4 * k + 3] != 0.f ? 0x1000000u : 0u);
-                for (int h = 0; h < sig; ++h) {
-                    uint32_t q[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) q[k] = h == c ? r[k] : 0u;
-                    ln_tmem_st8(tA + 16u * (uint32_t)h + 8u * (uint32_t)j, q);
-                }
-            } else {
-                uint32_t r[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) r[k] = pn_pack2<FP16>(v[2 * k], v[2 * k + 1]);
-                for (int h = 0; h < sig; ++h) {
-                    uint32_t q[16];
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) q[k] = h == c ? r[k] : 0u;
-                    pn_tmem_st16(tA + 32u * (uint32_t)h + 16u * (uint32_t)j, q);
-                }
-            }
-        };
-        auto start_chunk = [&](int j, float (&v)[32]) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float s0 = s_start[32 * j + i];
-                v[i] = live ? (BOOL ? (s0 != 0.f ? 1.f : 0.f) : s0) : 0.f;
-            }
-        };
+        const uint32_t FULL = 0xffffffffu;
+        uint32_t d[64];   // this string's states: a row of D
         auto d_value = [&](uint32_t w) -> float {
             if constexpr (I8) return w != 0u ? 1.f : 0.f;
             else if constexpr (BOOL) return __uint_as_float(w) > 0.f ? 1.f : 0.f;
             else return __uint_as_float(w);
         };
+        // this string's A row: the states in the K range of symbol c, zeros in the other ranges
+        // (tcgen05.st is warp-wide; each thread supplies its own row)
+        auto store_row = [&]() {
+            if constexpr (I8) {
+                uint32_t r[16];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            float v[32];
-            start_chunk(j, v);
-            store_chunk(j, v);
-        }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        pn_tc_before();
-        const uint32_t FULL = 0xffffffffu;
-        for (uint32_t ph = 0;; ph ^= 1u) {
-            const uint32_t any_live = __any_sync(FULL, live) ? 1u : 0u;
-            if (lane == 0) {
-                *reinterpret_cast<volatile uint32_t *>(&s_alive[T][ph][qd]) = any_live;
-                pn_mbar_arrive(bar_ready);
+                for (int k = 0; k < 16; ++k) {
+                    // four path counts (at most 64 each) as bytes, then 1 for each that is not 0
+                    const uint32_t w = __byte_perm(__byte_perm(d[4 * k], d[4 * k + 1], 0x0040),
+                                                   __byte_perm(d[4 * k + 2], d[4 * k + 3], 0x0040), 0x5410);
+                    r[k] = ((w + 0x7F7F7F7Fu) >> 7) & 0x01010101u;
+                }
+                for (int h = 0; h < sig; ++h) {
+                    uint32_t q[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) q[k] = h == c ? r[k] : 0u;
+                    pn_tmem_st16(tA + 16u * (uint32_t)h, q);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    uint32_t r[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k)
+                        r[k] = pn_pack2<FP16>(d_value(d[32 * j + 2 * k]), d_value(d[32 * j + 2 * k + 1]));
+                    for (int h = 0; h < sig; ++h) {
+                        uint32_t q[16];
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) q[k] = h == c ? r[k] : 0u;
+                        pn_tmem_st16(tA + 32u * (uint32_t)h + 16u * (uint32_t)j, q);
+                    }
+                }
             }
-            __syncwarp();
-            // all four warps of the tile have arrived: their flags decide whether it goes on
-            if (!pn_wait_park(bar_ready, ph, abort_flag, P.err, P.wait_cycles)) break;
-            const volatile uint32_t *fl = s_alive[T][ph];
-            if ((fl[0] | fl[1] | fl[2] | fl[3]) == 0u) break;
-            if (!pn_wait_park(bar_full, ph, abort_flag, P.err, P.wait_cycles)) break;
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            pn_tc_before();
+        };
+        // d becomes the start vector (zeros without a string) where `fresh`
+        auto start_row = [&](bool fresh) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i) {
+                const float s0 = s_start[i];
+                const uint32_t w = !live ? 0u : I8 ? (s0 != 0.f ? 1u : 0u)
+                                              : __float_as_uint(BOOL ? (s0 != 0.f ? 1.f : 0.f) : s0);
+                if (fresh) d[i] = w;
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < 64; ++i) d[i] = 0u;
+        start_row(true);
+        __syncwarp();
+        store_row();
+        uint32_t ph = 0u;
+        bool failed = false, pend = false;
+        for (;;) {
+            if (!ln_tile_any(T, live)) break;
+            if (failed) continue;   // (the other warps of the tile give up at their next wait)
             pn_tc_after();
-            // D row = this string's state after its symbol; what comes next
+            if (qd == 0) {
+                // One K chain (4 sigma K16 or 2 sigma K32 steps), issued by an elected thread with
+                // the steps unrolled: 37-43 cycles an MMA (M = 128, N = 64, K = 16 takes 32); a loop
+                // under `lane == 0` moves every operand to a uniform register: 103-109.
+                if (ln_elect()) {
+                    // K step kk: B 2 kLnLbo bytes further (+128 in the descriptor's start field,
+                    // which stays below 2^14 for shared addresses), A 8 TMEM columns further
+                    constexpr int KS = I8 ? 2 : 4;
+                    for (int h = 0; h < sig; ++h) {
+#pragma unroll
+                        for (int k = 0; k < KS; ++k) {
+                            const uint32_t kk = (uint32_t)(KS * h + k);
+                            const uint64_t desc = desc0 + (uint64_t)(128u * kk);
+                            const uint32_t ta = tile + 8u * kk, td = tile + P.a_cols;
+                            const uint32_t acc = kk > 0u;
+                            if constexpr (I8)
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                                    :: "r"(td), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
+                            else
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                                    :: "r"(td), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
+                        }
+                    }
+                    asm volatile(
+                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                        :: "r"(bar_full) : "memory");
+                }
+                __syncwarp();
+            }
+            pend = true;
+            // while the products run: what comes after this symbol
             const int nc = live ? ln_next(sy, sig, lo, hi) : -1;
             const bool ending = live && nc < 0;
             bool resc_now = false;
@@ -438,144 +492,61 @@ __global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(LnParams P) {
                     resc_now = true;
                 }
             }
-            bool from_d = live && !ending;
-            float sc = 1.f;
-            if (__any_sync(FULL, ending || resc_now)) {   // pass 1: the row's maximum, accept sum
-                float m = 0.f, dot = 0.f;
+            if (!ln_wait(bar_full, ph, abort_flag, P.err, P.wait_cycles)) {
+                failed = true;
+                live = false;
+                continue;
+            }
+            ph ^= 1u;
+            pend = false;
+            pn_tc_after();
+            // D row = this string's state after its symbol
+            ln_tmem_ld32(tD, d);
+            ln_tmem_ld32(tD + 32u, d + 32);
+            ln_tmem_wait32(d);
+            ln_tmem_wait32(d + 32);
+            const bool any_end = __any_sync(FULL, ending);
+            if (any_end) {   // a string's last symbol: the accept-weighted sum of its state
+                float dot = 0.f;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    uint32_t d[32];
-                    ln_tmem_ld32(tD + 32u * (uint32_t)j, d);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const float v = d_value(d[i]);
-                        m = fmaxf(m, fabsf(v));
-                        dot = fmaf(s_acc[32 * j + i], v, dot);
-                    }
-                }
+                for (int i = 0; i < 64; ++i) dot = fmaf(s_acc[i], d_value(d[i]), dot);
                 if (ending) {   // the string's log-likelihood, then the next string
                     ln_finish(P, seq, dot, E);
                     live = fetch();
                     E = 0;
                     since = 0;
-                } else if (resc_now) {   // exact power-of-two rescale
-                    int f = pn_ceil_exp(m);
-                    f = min(max(f, -125), 125);
-                    sc = pn_pow2(-f);
-                    E += f;
-                }
-            }
-            if (!live) c = 0;
-            // pass 2: the next A row, 32 states at a time
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                uint32_t d[32];
-                ln_tmem_ld32(tD + 32u * (uint32_t)j, d);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if constexpr (I8) {   // 0/1 bytes straight from the int32 path counts
-                    uint32_t r[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        r[k] = from_d ? ((d[4 * k] != 0u ? 1u : 0u) | (d[4 * k + 1] != 0u ? 0x100u : 0u) |
-                                         (d[4 * k + 2] != 0u ? 0x10000u : 0u) |
-                                         (d[4 * k + 3] != 0u ? 0x1000000u : 0u))
-                                      : (live ? s_start8[8 * j + k] : 0u);
-                    for (int h = 0; h < sig; ++h) {
-                        uint32_t q[8];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) q[k] = h == c ? r[k] : 0u;
-                        ln_tmem_st8(tA + 16u * (uint32_t)h + 8u * (uint32_t)j, q);
-                    }
-                    continue;
-                }
-                float v[32];
-                if (from_d) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = d_value(d[i]) * sc;
-                } else {
-                    start_chunk(j, v);
-                }
-                store_chunk(j, v);
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            pn_tc_before();
-        }
-    } else if (warp >= kLnEpiWarps) {
-        // MMA issuers: each its tiles round robin, one K chain (4 sigma K16 or 2 sigma K32 steps)
-        // each (two issuing threads: one alone spends ~135 cycles an instruction)
-        const uint32_t fmt = KIND == 1 ? 0u : 1u;
-        const uint32_t idesc = I8 ? ((2u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24))
-                                  : ((1u << 4) | (fmt << 7) | (fmt << 10) | ((64u >> 3) << 17) |
-                                     ((128u >> 4) << 24));
-        const uint32_t sb = pn_smem_u32(s_b);
-        const uint64_t desc0 = (uint64_t)(((sb >> 4) & 0x3FFFu) | ((kLnLbo >> 4) << 16)) |
-                               ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
-        const int nk = I8 ? 2 * sig : 4 * sig;
-        const int mw = warp - kLnMmaWarp;
-        uint32_t done = 0u, phs = 0u, pend = 0u;
-        for (int T = 0; T < kLnTiles; ++T)
-            if (T % kLnMmaWarps != mw || T >= P.tiles) done |= 1u << T;
-        bool aborted = false;
-        while (done != (1u << kLnTiles) - 1u && !aborted) {
-            for (int T = mw; T < kLnTiles; T += kLnMmaWarps) {
-                if ((done >> T) & 1u) continue;
-                if (!pn_wait_park(pn_smem_u32(&s_bar[kLnTiles + T]), (phs >> T) & 1u, abort_flag, P.err, P.wait_cycles)) {
-                    aborted = true;
-                    break;
-                }
-                pn_tc_after();
-                const volatile uint32_t *fl = s_alive[T][(phs >> T) & 1u];
-                phs ^= 1u << T;
-                pend &= ~(1u << T);   // the epilogue has read the previous product
-                if ((fl[0] | fl[1] | fl[2] | fl[3]) == 0u) {
-                    done |= 1u << T;
-                    continue;
-                }
-                if (lane == 0) {
-                    // K step kk: B 2 kLnLbo bytes further (+128 in the descriptor's start field,
-                    // which stays below 2^14 for shared addresses), A 8 TMEM columns further
-                    const uint32_t tA = tbase + (uint32_t)T * P.tile_cols, tD = tA + P.a_cols;
-                    for (int kk = 0; kk < nk; ++kk) {
-                        const uint64_t desc = desc0 + (uint64_t)(128u * (uint32_t)kk);
-                        const uint32_t ta = tA + 8u * (uint32_t)kk;
-                        const uint32_t acc = kk > 0;
-                        if constexpr (I8)
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-                                :: "r"(tD), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
-                        else
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                                :: "r"(tD), "r"(ta), "l"(desc), "r"(idesc), "r"(acc) : "memory");
-                    }
-                    asm volatile(
-                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                        :: "r"(pn_smem_u32(&s_bar[T])) : "memory");
                 }
                 __syncwarp();
-                pend |= 1u << T;
             }
+            if (!BOOL && __any_sync(FULL, resc_now)) {   // exact power-of-two rescale by the row's maximum
+                float m = 0.f;
+#pragma unroll
+                for (int i = 0; i < 64; i += 2) m = ln_max_abs3(m, __uint_as_float(d[i]), __uint_as_float(d[i + 1]));
+                const int f = resc_now ? min(max(pn_ceil_exp(m), -125), 125) : 0;
+                const float sc = pn_pow2(-f);
+                E += f;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) d[i] = __float_as_uint(__uint_as_float(d[i]) * sc);
+            }
+            if (!live) c = 0;
+            // (the row of a lane without a string stays zero)
+            if (any_end) start_row(ending);
+            __syncwarp();
+            store_row();
         }
         // a product committed but not read must be complete before the TMEM is freed
-        for (int T = 0; T < kLnTiles; ++T) {
-            if (!((pend >> T) & 1u)) continue;
-            if (lane == 0) {
-                const uint32_t par = ((phs >> T) & 1u) ^ 1u;   // the phase of the last commit
-                const long long t0 = clock64();
-                while (!pn_mbar_test(pn_smem_u32(&s_bar[T]), par)) {
-                    if (clock64() - t0 > kPnDrainCycles) { atomicOr(P.err, kPnErrTimeout); break; }
-                }
+        if (qd == 0 && pend && lane == 0) {
+            const long long t0 = clock64();
+            while (!pn_mbar_test(bar_full, ph)) {
+                if (clock64() - t0 > kPnDrainCycles) { atomicOr(P.err, kPnErrTimeout); break; }
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     pn_tc_before();
     __syncthreads();
     pn_tc_after();
-    if (warp == kLnMmaWarp)
+    if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(512));
 }
 
@@ -1120,7 +1091,10 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
         TREX_CHECK_LAUNCH();
         return TREX_OK;
     }
-    if (h->sigma <= kLnMaxSigma) {   // strings on TMEM lanes, no sorting by symbol (sigma <= 4)
+    // Strings on TMEM lanes up to four symbols: at four, 262144 x 512 take 4.26 / 4.65 / 2.53 ms (BF16,
+    // FP16, int8) there and 7.11 / 8.94 / 5.30 with lists by symbol; above, A's columns (32 a symbol)
+    // leave room for fewer tiles and B outgrows its 32 KB.
+    if (h->sigma <= kLnMaxSigma) {
         const int k = mode == TREX_PNFA_FP16 ? 1 : mode == TREX_PNFA_BOOL8 ? 2 : mode == TREX_PNFA_BOOL ? 3 : 0;
         LnParams Q;
         Q.data = data;
