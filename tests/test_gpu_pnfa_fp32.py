@@ -80,3 +80,28 @@ def test_fp32_hand_off_gives_up(cuda):
     torch.cuda.synchronize()
     assert m.error_word() == 0 and bool(torch.isfinite(ll).all())
     m.close()
+
+
+def test_fp32_long_skipped_runs_are_work(cuda, oracle):
+    # runs of 16 MiB outside the alphabet, at a string's start and inside it, take many times the
+    # wait limit set here; skipping is not a stalled hand-off
+    from trex_b200 import _lib
+    rng = np.random.default_rng(8)
+    T, start, acc = (x.astype(np.float32) for x in random_prob_nfa(rng, 64, 20))
+    run, tail = 16 << 20, 37
+    off = np.array([0, run + tail, 2 * run + 2 * tail, 2 * run + 2 * tail + 500], dtype=np.int64)
+    data = np.full(int(off[-1]), 200, dtype=np.uint8)
+    data[run:run + tail] = rng.integers(0, 20, size=tail)                  # skipped bytes first
+    data[off[1]:off[1] + 9] = rng.integers(0, 20, size=9)                  # between symbols
+    data[off[2] - 21:off[2] - 1] = rng.integers(0, 20, size=20)            # (and one at the end)
+    data[off[2]:] = rng.integers(0, 20, size=500)
+    lib = _lib.load()
+    try:
+        _lib.check(lib.trex_set_wait_limits(0, 4_000_000), "trex_set_wait_limits")
+        ll, ac, err = _run(cuda, T, start, acc, data, off)
+    finally:
+        _lib.check(lib.trex_set_wait_limits(0, 0), "trex_set_wait_limits")
+    assert err == 0
+    ref = oracle.pnfa_fp64(T, start, acc, data, off)
+    assert np.all(np.abs(ll - ref) <= 1e-5 * np.abs(ref))   # at most 500 symbols, as above
+    assert np.array_equal(ac.astype(bool), ref > np.log(0.5))

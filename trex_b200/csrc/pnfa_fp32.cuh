@@ -55,6 +55,7 @@ struct RiParams {
 // Shared memory: control words, rings (n_rings, then that of ended slots), records, state rows,
 // tables.
 constexpr uint32_t kRiTails = 0;                        // uint32 [kRiWarps + 1]
+constexpr uint32_t kRiSkips = 4 * (kRiWarps + 1);       // pieces of skipped bytes (ri_skip)
 constexpr uint32_t kRiEndHead = 128, kRiLock = 132, kRiLive = 136, kRiDone = 140;
 constexpr uint32_t kRiAcc = 144;                        // float [64]
 constexpr uint32_t kRiStart = kRiAcc + 256;             // uint4 [16]
@@ -134,6 +135,38 @@ __device__ __forceinline__ uint32_t ri_poll(const RiParams &P, uint32_t ring, ui
     return got == 0xffffffffu ? 32u : (uint32_t)__ffs(~got) - 1u;
 }
 
+// The first byte below sigma of [p, e), or e: 64 bytes a step, so that a long run of skipped
+// bytes does not take a round trip a byte. Every piece of 4 KiB counts as work done (ri_stalled).
+__device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_t *e, uint32_t sigma) {
+    const uint32_t sig4 = sigma * 0x01010101u;
+    while (p < e && (reinterpret_cast<uintptr_t>(p) & 15u)) {
+        if (__ldg(p) < sigma) return p;
+        ++p;
+    }
+    for (uint32_t steps = 1; e - p >= 64; p += 64, ++steps) {
+        uint32_t in = 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p) + k);
+            in |= __vcmpltu4(v.x, sig4) | __vcmpltu4(v.y, sig4) | __vcmpltu4(v.z, sig4) | __vcmpltu4(v.w, sig4);
+        }
+        if (in) break;
+        if (steps % 64u == 0u) ri_add32(ri_base() + kRiSkips, 1u);
+    }
+    while (p < e && __ldg(p) >= sigma) ++p;
+    return p;
+}
+// The next symbol of a slot's string (its record at rec), 255 at its end; moves the record on.
+// Not inlined: the tables stay in registers.
+__device__ __noinline__ uint32_t ri_next(uint32_t rec, uint32_t sigma) {
+    const uint8_t *p, *e;
+    ri_ldp(rec + kRiRecP, p, e);
+    p = ri_skip(p, e, sigma);
+    if (p == e) return 255u;
+    ri_stp(rec + kRiRecP, p + 1);
+    return __ldg(p);
+}
+
 // Gives a slot the next string of the batch: its record, its start row and its first ring.
 // Strings without symbols get their result at once; false when the batch has no more strings.
 __device__ __forceinline__ bool ri_refill(const RiParams &P, uint32_t slot) {
@@ -146,8 +179,8 @@ __device__ __forceinline__ bool ri_refill(const RiParams &P, uint32_t slot) {
             continue;
         }
         const uint8_t *p = P.data + p0, *const e = P.data + p1;
-        uint32_t c = 255u;
-        while (p < e && (c = __ldg(p)) >= (uint32_t)P.sigma) ++p;
+        uint32_t c = p < e ? __ldg(p) : 255u;
+        if (c >= (uint32_t)P.sigma && p < e && (p = ri_skip(p + 1, e, (uint32_t)P.sigma)) < e) c = __ldg(p);
         if (p == e) {
             pn_write_result(P.loglik, P.accept, P.accept_i32, (int64_t)idx, P.ll_empty);
             continue;
@@ -203,12 +236,13 @@ __device__ __forceinline__ bool ri_try_feed(const RiParams &P, uint32_t least) {
     return true;
 }
 
-// A wait without work: true when nothing moved in any ring for `limit` clock cycles (all lanes
-// call it; mark and t0 carry over between calls).
+// A wait without work: true when nothing moved in any ring, and no lane skipped on in its string,
+// for the limit of clock cycles (all lanes call it; mark and t0 carry over between calls).
 __device__ __forceinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
     const uint32_t lane = threadIdx.x & 31u;
     if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) return false;
-    const uint32_t v = (int)lane <= P.n_rings ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
+    const bool counts = (int)lane <= P.n_rings || lane == (kRiSkips - kRiTails) / 4u;
+    const uint32_t v = counts ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
     const uint32_t sum = __reduce_add_sync(0xffffffffu, v);
     if (sum == mark) return true;
     mark = sum;
@@ -219,7 +253,7 @@ __device__ __forceinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, lo
 // Waits for entries of a ring (up to `most`), feeding ended slots meanwhile; 0 when the work is
 // done (or the wait gave up).
 __device__ __forceinline__ uint32_t ri_wait(const RiParams &P, uint32_t ring, uint32_t head, uint32_t most, uint32_t &ent) {
-    uint32_t cnt, mark = 0u;
+    uint32_t cnt, mark = 0xFFFFFFFFu;   // (no sum yet)
     long long t0 = 0;
     ri_try_feed(P, 32u);
     while ((cnt = ri_poll(P, ring, head, most, ent)) == 0u) {
@@ -333,14 +367,10 @@ __global__ void __launch_bounds__(kRiThreads, 1) pnfa_fp32_kernel(const __grid_c
         if (own) {   // the symbol after this one (bytes >= sigma are skipped)
             const uint8_t *p, *e;
             ri_ldp(rec + kRiRecP, p, e);
-            bool found = p < e && nc < (uint32_t)P.sigma;
-            if (p < e) ++p;
-            while (!found && p < e) {
-                nc = __ldg(p++);
-                found = nc < (uint32_t)P.sigma;
-            }
-            ending = !found;
-            ri_stp(rec + kRiRecP, p);
+            const bool found = p < e && nc < (uint32_t)P.sigma;
+            if (p < e) ri_stp(rec + kRiRecP, ++p);
+            if (!found) nc = p < e ? ri_next(rec, (uint32_t)P.sigma) : 255u;
+            ending = nc >= (uint32_t)P.sigma;
         }
         const uint32_t ends = __ballot_sync(FULL, ending);
 #pragma unroll
