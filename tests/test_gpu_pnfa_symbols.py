@@ -95,3 +95,24 @@ def test_growing_states_are_rescaled(cuda, oracle):
             ll, ac, err = _run(cuda, T, start, acc, data, off, mode)
             assert err == 0
             _check(oracle, T, start, acc, data, off, mode, ll, ac)
+
+
+def test_int8_tables_of_two_symbols_a_warp_stay_in_registers(cuda):
+    # one symbol more than warps costs the eight-string groups of a second list, not a table's
+    # load a step (which was 22 times the time of 20 symbols)
+    from trex_b200.engine import PNFA
+    ms = {}
+    for sigma in (20, 21):
+        rng = np.random.default_rng(sigma)
+        m = PNFA(*_automaton(rng, 64, sigma, "bool8"))
+        off = cuda.arange(0, 8193, dtype=cuda.int64, device="cuda") * 256
+        data = cuda.from_numpy(rng.integers(0, sigma, size=8192 * 256, dtype=np.uint8)).cuda()
+        for _ in range(6):
+            t0, t1 = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+            t0.record()
+            m.run(data, off, "bool8")
+            t1.record()
+            t1.synchronize()
+            ms[sigma] = min(ms.get(sigma, 1e9), t0.elapsed_time(t1))
+        m.close()
+    assert ms[21] < 4 * ms[20], ms

@@ -422,23 +422,25 @@ __device__ __forceinline__ void sy_group(const SyParams &P, const uint32_t (&a)[
 
 // A warp's groups of step t; mine: its symbol, and the first group it takes of the symbol's list
 // (in the upper half).
-template <int KIND, bool SEVERAL, bool SCALE, bool MAX>
+template <int KIND, bool RELOAD, bool SCALE, bool MAX>
 __device__ __forceinline__ void sy_groups(const SyParams &P, uint32_t (&a)[4][KIND == 2 ? 2 : 4][4], uint32_t t,
                                           uint32_t mine) {
     for (uint32_t c = mine & 0xFFFFu; c < (uint32_t)P.sigma; c += blockDim.x >> 5) {
         int n = (int)sy_at<uint32_t>(kSyCnt + 128u * (t % 3u) + 4u * c);
-        if (SEVERAL && n != 0) sy_load_table<KIND>(P, (int)c, a);
+        if (RELOAD && n != 0) sy_load_table<KIND>(P, (int)c, a);
         const float R = SCALE ? __ldg(P.rsym + c) : 0.f;
-        const uint32_t first = SEVERAL ? 0u : mine >> 16, step = SEVERAL ? 8u : 8u * (uint32_t)P.rep;
+        const uint32_t first = RELOAD ? 0u : mine >> 16, step = RELOAD ? 8u : 8u * (uint32_t)P.rep;
         uint32_t ent = P.list_off + (2u << P.cap_shift) * ((t & 1u) * (uint32_t)P.sigma + c) + 2u * first;
         for (n -= (int)first; n > 0; n -= (int)step, ent += 2u * step)
             sy_group<KIND, SCALE, MAX>(P, a, ent, (uint32_t)min(8, n), R, t);
-        if (!SEVERAL) break;
+        if (!RELOAD) break;
     }
 }
 
-// SEVERAL: alphabets of more symbols than warps; a warp loads its symbols' tables in turn at
-// every step.
+// SEVERAL: alphabets of more symbols than warps. Two int8 tables take the registers of one in 16
+// bits, so a warp keeps both (8192 strings x 512, 20 / 21 / 28 symbols: 0.53 / 0.83 / 0.91 ms; loading
+// each table at every step, 12.0 / 14.5 for 21 / 28); in the 16-bit forms it loads its symbols' tables in
+// turn at every step (BF16 0.73 / 2.09 / 2.35, FP16 0.84 / 2.14 / 2.41).
 template <int KIND, bool SEVERAL>
 __global__ void __launch_bounds__(kSyThreads, 1) pnfa_sym_kernel(const __grid_constant__ SyParams P) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -447,9 +449,11 @@ __global__ void __launch_bounds__(kSyThreads, 1) pnfa_sym_kernel(const __grid_co
     if (threadIdx.x < 8) sy_at<uint4>(kSyStart + 16u * threadIdx.x) = P.start_img[threadIdx.x];
     for (uint32_t s = threadIdx.x; s < (uint32_t)P.slots; s += blockDim.x) sy_at<uint8_t>(P.state_off + s) = (uint8_t)kSlFree;
     __syncthreads();
-    uint32_t a[4][KIND == 2 ? 2 : 4][4];
+    constexpr bool BOTH = SEVERAL && KIND == 2, RELOAD = SEVERAL && !BOTH;
+    uint32_t a[4][KIND == 2 ? 2 : 4][4], a2[4][KIND == 2 ? 2 : 4][4];   // (a2: with BOTH)
     const uint32_t mine = warp % (uint32_t)P.sigma | ((8u * (warp / (uint32_t)P.sigma)) << 16);
-    if (!SEVERAL) sy_load_table<KIND>(P, (int)(mine & 0xFFFFu), a);
+    if (!RELOAD) sy_load_table<KIND>(P, (int)(mine & 0xFFFFu), a);
+    if (BOTH && warp + kSyWarps < (uint32_t)P.sigma) sy_load_table<KIND>(P, (int)(warp + kSyWarps), a2);
     for (uint32_t t = 0;; ++t) {
         // meetings before this step's: one a step and one a block
         if (t % kSyBlk == 0u) {
@@ -467,14 +471,15 @@ __global__ void __launch_bounds__(kSyThreads, 1) pnfa_sym_kernel(const __grid_co
         // (the lengths of the step after the next: read by nobody in this step)
         if (threadIdx.x < 32u) sy_at<uint32_t>(kSyCnt + 128u * ((t + 2u) % 3u) + 4u * lane) = 0u;
         if (KIND >= 2) {
-            sy_groups<KIND, SEVERAL, false, false>(P, a, t, mine);
+            sy_groups<KIND, RELOAD, false, false>(P, a, t, mine);
+            if constexpr (BOTH) sy_groups<KIND, false, false, false>(P, a2, t, warp + kSyWarps);
         } else if (P.resc == 1) {
-            sy_groups<KIND, SEVERAL, true, true>(P, a, t, mine);
+            sy_groups<KIND, RELOAD, true, true>(P, a, t, mine);
         } else {
             const uint32_t x = t & (uint32_t)(P.resc - 1);
-            if (x == 0u) sy_groups<KIND, SEVERAL, true, false>(P, a, t, mine);
-            else if (x + 1u == (uint32_t)P.resc) sy_groups<KIND, SEVERAL, false, true>(P, a, t, mine);
-            else sy_groups<KIND, SEVERAL, false, false>(P, a, t, mine);
+            if (x == 0u) sy_groups<KIND, RELOAD, true, false>(P, a, t, mine);
+            else if (x + 1u == (uint32_t)P.resc) sy_groups<KIND, RELOAD, false, true>(P, a, t, mine);
+            else sy_groups<KIND, RELOAD, false, false>(P, a, t, mine);
         }
         if (!sy_meet(P, t + t / kSyBlk + 1u)) break;
     }
