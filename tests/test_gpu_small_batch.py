@@ -88,6 +88,57 @@ def test_small_batch_automata_that_never_synchronise(cuda, oracle, n_states, len
     assert np.array_equal(fs, _expect(oracle, [dfa], data, off, np.zeros(len(lens), dtype=int)))
 
 
+def _keep_state_dfa(n):
+    """No byte changes the state: only the lane beside the start is wrong, then the next one."""
+    acc = np.zeros(n, dtype=np.uint8)
+    acc[n - 1] = 1
+    return ByteDFA(n_states=n, tmap=np.tile(np.arange(n, dtype=np.uint8), 256), accept=acc, start=n - 1)
+
+
+# state maps of whole pieces: shares of 8 to 256 states, one piece, odd ends, many pieces
+@pytest.mark.parametrize("n_states", [1, 2, 8, 9, 16, 17, 100, 129, 256])
+@pytest.mark.parametrize("make", [_permutation_dfa, lambda n, rng: _keep_state_dfa(n)], ids=["permutes", "keeps"])
+def test_small_batch_pieces_as_state_maps(cuda, oracle, n_states, make):
+    rng = np.random.default_rng(n_states)
+    dfas = [make(n_states, rng), random_dfa(5, np.arange(256), rng)]
+    lens = np.array([16385, 32768, 32769, 70001, 400, 16000, 131072 + 5, 900, 300003], dtype=np.int64)
+    data, off = _batch(lens, rng, lead=13)
+    ids = np.array([0, 0, 0, 0, 0, 0, 0, 1, 0])
+    from trex_b200.engine import DFASet
+    s = DFASet(dfas)
+    fs, ac, ai, err = _run(cuda, s, data, off, ids, 0)
+    assert err == 0
+    assert np.array_equal(fs, _expect(oracle, dfas, data, off, ids))
+    assert np.array_equal(ac, ai) and np.array_equal(ac, [dfas[d].accept[f] for d, f in zip(ids, fs)])
+    every, _ = s.run_all(cuda.from_numpy(data).cuda(), cuda.from_numpy(off).cuda())
+    s.close()
+    for d in (0, 1):
+        assert np.array_equal(every[d].cpu().numpy(), _expect(oracle, dfas, data, off, np.full(len(lens), d)))
+
+
+# The one launch may not cost automata that never synchronise what it saves the others: against the
+# planned path on the same batch (the forms differ by far more than the tolerance where one degenerates).
+@pytest.mark.parametrize("n_states", [8, 24, 100, 256])
+@pytest.mark.parametrize("shape", [(30, 100000), (200, 40000), (8000, 1000)])
+def test_small_batch_never_synchronising_is_not_slower(cuda, n_states, shape):
+    torch = cuda
+    from trex_b200.engine import DFASet
+    rng = np.random.default_rng(n_states)
+    s = DFASet([_permutation_dfa(n_states, rng)])
+    data, off = (torch.from_numpy(x).cuda() for x in _batch(np.full(shape[0], shape[1]), rng))
+    best = {}
+    for seg in (0, 2048, 0, 2048):
+        for _ in range(6):
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            t0.record()
+            s.run(data, off, seg_len=seg)
+            t1.record()
+            t1.synchronize()
+            best[seg] = min(best.get(seg, 1e9), t0.elapsed_time(t1))
+    s.close()
+    assert best[0] <= 1.5 * best[2048], best
+
+
 def test_small_batch_every_automaton(cuda, oracle):
     torch = cuda
     rng = np.random.default_rng(3)

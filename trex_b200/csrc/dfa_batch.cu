@@ -1934,20 +1934,23 @@ static int dfa_set_run_ex(trex_dfa_set *set, const uint8_t *data, const int64_t 
     // bytes, 16 KiB / 1 / 4 / 8 / 16 MiB: 14 / 15 / 19 / 27 / 37 against 86 / 78 / 101 / 116 / 117;
     // log-normal strings (median 512): 15 / 33 / 44 / 62 / 83 against 125 / 126 / 147 / 162 / 188;
     // 16 automata, strings of 64 bytes, 4 / 8 / 16 MiB: 33 / 58 / 108 against 69 / 74 / 84, so
-    // the limits lie at 8 MiB and as many strings as 64-byte ones make.
-    if (seg_len_in <= 0 && n <= kSmallStrings && walked <= kSmallBytes) {
-        const bool in_smem = set->tmap_bytes <= kSmallMapBytes;
-        P.fix_tm_bytes = in_smem ? (uint32_t)set->tmap_bytes : 0u;
+    // the limits lie at 8 MiB and as many strings as 64-byte ones make. Sets whose maps do not fit in
+    // shared memory are planned (64 automata of 64 states, 8000 strings of 1000 bytes: 220 read from
+    // L2 against 124).
+    if (seg_len_in <= 0 && n <= kSmallStrings && walked <= kSmallBytes && set->tmap_bytes <= kSmallMapBytes) {
+        P.fix_tm_bytes = (uint32_t)set->tmap_bytes;
         const int grid = (int)std::min<int64_t>(
             set->n_sms, std::max<int64_t>((n + 7) / 8, walked / (32 * kSmallPieceWindows)));
-        // report counters and records of long strings, in the room for work items (32 bytes for
-        // every 2048 bytes of the batch; at most 8 for every kSmallLongBytes here)
-        uint32_t *cnt = reinterpret_cast<uint32_t *>(items);
+        // Report counters and records of long strings lie in the room for item results (8 bytes for every
+        // string and every 2048 bytes walked), the pieces' state maps in that for work items (32 bytes for
+        // each: a string above kSmallLongBytes has room for one map, one of several pieces for 256 bytes a
+        // piece).
+        uint32_t *cnt = reinterpret_cast<uint32_t *>(maps);
         const int64_t max_long = walked / kSmallLongBytes + 1;
         if (max_long > 1) TREX_CUDA(cudaMemsetAsync(cnt, 0, (size_t)max_long * 4, stream));
+        uint8_t *const st_maps = reinterpret_cast<uint8_t *>(items);
         profile_kernel_begin(stream);
-        if (in_smem) dfa_small_kernel<true><<<grid, kSmallThreads, set->tmap_bytes, stream>>>(P, cnt, cnt + max_long);
-        else dfa_small_kernel<false><<<grid, kSmallThreads, 0, stream>>>(P, cnt, cnt + max_long);
+        dfa_small_kernel<<<grid, kSmallThreads, set->tmap_bytes, stream>>>(P, cnt, cnt + max_long, st_maps);
         TREX_CHECK_LAUNCH();
         profile_kernel_end(stream);
         if (err_word_out) *err_word_out = err;
@@ -2095,7 +2098,7 @@ int trex_dfa_set_create(int n_dfas, const int32_t *n_states, const int32_t *star
     if ((e = cudaFuncSetAttribute(trex::compose_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)trex::kFixSmemBytes)) != cudaSuccess)
         return fail(e, "cudaFuncSetAttribute");
-    if ((e = cudaFuncSetAttribute(trex::dfa_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if ((e = cudaFuncSetAttribute(trex::dfa_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)trex::kSmallMapBytes)) != cudaSuccess)
         return fail(e, "cudaFuncSetAttribute");
     *out = set;
