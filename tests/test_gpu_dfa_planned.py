@@ -46,3 +46,30 @@ def test_tables_of_each_layout(cuda, oracle, n_states):
     data = rng.integers(0, 256, size=int(off[-1]), dtype=np.uint8)
     ids = rng.integers(0, 2, size=4000).astype(np.int32)
     _check(cuda, oracle, dfas, data, off, ids, 256)
+
+
+# Queues shared out to a CTA's warps: fewer batches than CTAs, one more than a share, one automaton
+# with most of the items among many with a few, letters of 16 (32 items a claim), large automata.
+@pytest.mark.parametrize("case", ["one_short", "a_share_and_one", "uneven", "letters", "large"])
+def test_short_queues(cuda, oracle, case):
+    from trex_b200.engine import DFASet
+    rng = np.random.default_rng(len(case))
+    letters = np.arange(65, 81, dtype=np.uint8)
+    sizes, n = {"one_short": ([40], 50), "a_share_and_one": ([16], 64 * 149), "uneven": ([8, 16, 64] * 20, 9000),
+                "letters": ([12], 9000), "large": ([100, 250, 7], 3000)}[case]
+    dfas = [random_dfa(k, letters if case == "letters" else np.arange(256), rng) for k in sizes]
+    lens = rng.integers(0, 3000, size=n)
+    off = np.zeros(n + 1, dtype=np.int64)
+    np.cumsum(lens, out=off[1:])
+    data = rng.integers(0, 256, size=int(off[-1]), dtype=np.uint8)
+    if case == "letters":
+        data = letters[data & 15]
+    ids = np.where(rng.random(n) < 0.7, 0, rng.integers(0, len(dfas), size=n)).astype(np.int32)
+    s = DFASet(dfas, kgram=0 if case == "letters" else None)
+    for seg in (512, 2048):
+        fs, ac, _ = s.run(*(cuda.from_numpy(x).cuda() for x in (data, off, ids)), seg_len=seg)
+        want, wacc = oracle.dfa_walk([d.tmap for d in dfas], [d.n_states for d in dfas], [0] * len(dfas),
+                                     [d.accept for d in dfas], data, off, ids)
+        assert s.last_error_word() == 0
+        assert np.array_equal(fs.cpu().numpy(), want) and np.array_equal(ac.cpu().numpy(), wacc)
+    s.close()

@@ -954,7 +954,8 @@ __device__ inline void build_gram_tables(const DfaDesc &D, const uint8_t *__rest
 constexpr uint32_t kLaneItemsOff = kFallbackOff + kFallbackBytes;
 // Then one 32-bit word a thread and chain: the checkpoints of the chain's item.
 constexpr uint32_t kCpOff = kLaneItemsOff + kRaggedThreads * 2 * (uint32_t)sizeof(WorkItem);
-constexpr uint32_t kRaggedSmemBytes = kCpOff + kRaggedThreads * 2 * 4;
+constexpr uint32_t kWarpsOff = kCpOff + kRaggedThreads * 2 * 4;   // uint32: warps that claim items
+constexpr uint32_t kRaggedSmemBytes = kWarpsOff + 16;
 
 // Checkpoints of an item after the first of its string: its chain's state at
 // the start of windows cw + 1, cw + 2, cw + 4 and cw + 8 (32, 64, 128 and 256
@@ -1120,6 +1121,17 @@ __device__ __forceinline__ void whole_windows(const M &md, uint32_t &it, uint32_
     }
 }
 
+// Warps of the CTA that claim items of its queue: all of them from a long queue (and each claims its
+// next batch ahead), an even share of a short one. Without a share the CTAs that reach a queue first
+// empty it, with 32 busy warps each that walk several times slower than one or two a CTA, and the
+// time depends on who comes first (32- and 64-state automata, 100003 log-normal strings, at four
+// addresses of the batch: 407-496 us a call; with shares 385-389; 9000 strings on 64 states, kernel:
+// 100-205 against 77; 1M strings on 16 automata: 1334 either way).
+__device__ __forceinline__ volatile uint32_t &claiming_warps() {
+    return *reinterpret_cast<volatile uint32_t *>(g_dfa_tbl + kWarpsOff);
+}
+__device__ __forceinline__ bool claims_ahead() { return claiming_warps() == kRaggedThreads / 32; }
+
 // Drains queue d with this warp, 32 items (one a lane, one chain a thread) at
 // a time; automata of at most 8 states take this path (their two-instruction
 // step gains nothing from a second chain on ragged batches, measured). The
@@ -1138,14 +1150,14 @@ __device__ void drain_queue_one(const RaggedParams &P, const M &md, const DfaDes
     const uint32_t FULL = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint8_t *const lo_ok = P.data, *const hi_ok = P.data + P.total_bytes;
-    uint32_t b0 = 0;
-    if (lane == 0) b0 = atomicAdd(head, 32u);
+    uint32_t b0 = count;
+    if (lane == 0 && (threadIdx.x >> 5) < claiming_warps()) b0 = atomicAdd(head, 32u);
     b0 = __shfl_sync(FULL, b0, 0);
     if (b0 >= count) return;
     WorkItem cur = load_item(P, base, b0 + lane, count);
     while (true) {
-        uint32_t b1 = 0;
-        if (lane == 0) b1 = atomicAdd(head, 32u);
+        uint32_t b1 = count;
+        if (lane == 0 && claims_ahead()) b1 = atomicAdd(head, 32u);
         b1 = __shfl_sync(FULL, b1, 0);
         const WorkItem nxt = load_item(P, base, b1 + lane, count);
 
@@ -1265,8 +1277,8 @@ __device__ void drain_queue(const RaggedParams &P, const M &md, const DfaDesc &D
     volatile uint32_t *const wv = s_warp[threadIdx.x >> 5];
     uint32_t *const slot0 = reinterpret_cast<uint32_t *>(g_dfa_tbl + kLaneItemsOff) + threadIdx.x;
     uint32_t *const slot1 = slot0 + 8 * kRaggedThreads;
-    uint32_t b0 = 0;
-    if (lane == 0) b0 = atomicAdd(&P.q_head[d], 64u);
+    uint32_t b0 = 0xffffffffu;
+    if (lane == 0 && (threadIdx.x >> 5) < claiming_warps()) b0 = atomicAdd(&P.q_head[d], 64u);
     b0 = __shfl_sync(FULL, b0, 0);
     {
         const uint32_t base = q_base_of(P, d), count = q_count_of(P, d);
@@ -1276,10 +1288,10 @@ __device__ void drain_queue(const RaggedParams &P, const M &md, const DfaDesc &D
     }
     while (true) {
         {
-            uint32_t b1 = 0;
-            if (lane == 0) b1 = atomicAdd(&P.q_head[d], 64u);
-            b1 = __shfl_sync(FULL, b1, 0);
             const uint32_t base = q_base_of(P, d), count = q_count_of(P, d);
+            uint32_t b1 = count;
+            if (lane == 0 && claims_ahead()) b1 = atomicAdd(&P.q_head[d], 64u);
+            b1 = __shfl_sync(FULL, b1, 0);
             if (b1 + lane < count) prefetch_l2(P.items + base + b1 + lane);
             if (b1 + 32 + lane < count) prefetch_l2(P.items + base + b1 + 32 + lane);
             __syncwarp();
@@ -1373,19 +1385,32 @@ __global__ void __launch_bounds__(kRaggedThreads, 1) dfa_ragged_kernel(RaggedPar
         unsigned long long tot = 0;
         for (int d = 0; d < P.n_dfas; ++d) tot += weight(d);
         int home = -1;
+        uint32_t warps = kRaggedThreads / 32;
         if (tot && planned) {
-            unsigned long long pos =
-                (unsigned long long)((double)tot * ((double)blockIdx.x + 0.5) / gridDim.x);
+            const double each = (double)tot / gridDim.x;
+            const unsigned long long pos = (unsigned long long)(each * ((double)blockIdx.x + 0.5));
             unsigned long long run = 0;
             for (int d = 0; d < P.n_dfas; ++d) {
-                run += weight(d);
-                if (P.q_count[d] && pos < run) { home = d; break; }
+                const unsigned long long w = weight(d);
+                const uint32_t count = P.q_count[d];
+                if (count && pos < run + w) {
+                    home = d;
+                    // the CTAs whose position lies in this queue's part share its batches
+                    const double ctas = ceil((double)(run + w) / each - 0.5) - ceil((double)run / each - 0.5);
+                    const bool one = P.desc[d].n_states <= 8 || (P.desc[d].kgram > 1 && P.desc[d].kbits == 4);
+                    const uint32_t per = one ? 32u : 64u;   // items a claim (see drain)
+                    if (count < 32u * per * (uint32_t)max(ctas, 1.0))
+                        warps = (uint32_t)ceil((double)((count + per - 1u) / per) / max(ctas, 1.0));
+                    break;
+                }
+                run += w;
             }
             if (home < 0)
                 for (int d = P.n_dfas - 1; d >= 0; --d)
                     if (P.q_count[d]) { home = d; break; }
         }
         if (home >= 0) atomicAdd(&P.q_serve[home], 1u);
+        claiming_warps() = warps;
         s_dfa = home;
     }
     __syncthreads();
@@ -1451,6 +1476,7 @@ __global__ void __launch_bounds__(kRaggedThreads, 1) dfa_ragged_kernel(RaggedPar
             }
             if (threadIdx.x == 0) {
                 if (best >= 0) atomicAdd(&P.q_serve[best], 1u);
+                claiming_warps() = kRaggedThreads / 32;
                 s_dfa = best;
             }
         }
