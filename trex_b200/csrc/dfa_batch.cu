@@ -290,24 +290,54 @@ __device__ __forceinline__ uint32_t warp_rank(uint32_t *cnt, bool pred, int key)
 }
 
 // The planning kernels run with the same grid of at most kMaxPlanCtas CTAs of
-// kPlanThreads threads, and a CTA takes the same tiles of kPlanThreads
-// consecutive strings in both: so the fill meets exactly the items the count
-// saw, and each CTA writes its items into a range of every queue class reserved
-// for it alone (no global atomics on the hot counters).
+// kPlanThreads threads, and a CTA takes the same strings in both: so the fill
+// meets exactly the items the count saw, and each CTA writes its items into a range of every
+// queue class reserved for it alone (no global atomics on the hot counters).
 //
-// A CTA's tiles are one contiguous share of the strings, because the order of a
-// class's items in its queue is the order in which the walk reads the buffer:
-// with tiles c, c + G, c + 2G, ... a warp's 64 items came from all over the
-// buffer, and the walk's streams were bound by address translation rather than
-// by bytes (1M log-normal strings, 4 GB, 16 automata, whole batch: 1391 us with
-// strided tiles, 1328 us with shares; streams of 2 KiB read in random order run at
-// 5.8 TB/s inside 128 MiB and at 1.4 TB/s inside 512 MiB).
-struct TileRange {
+// A CTA's strings are one contiguous share, because the order of a class's items in its queue is
+// the order in which the walk reads the buffer: with tiles of strings dealt out in turn a warp's 64
+// items came from all over the buffer, and the walk's streams were bound by address translation
+// rather than by bytes (1M log-normal strings, 4 GB, 16 automata, whole batch: 1391 us dealt out,
+// 1328 us with shares; streams of 2 KiB read in random order run at 5.8 TB/s inside 128 MiB and at
+// 1.4 TB/s inside 512 MiB). The shares of a large batch are equal in strings plus items, so that
+// one CTA does not list the items of all long strings where those lie together (the same batch with
+// its strings in order of length: 1297 us, equal numbers of strings 1420, dealt out 1310).
+struct StringRange {
     int64_t first, end;
 };
-__device__ __forceinline__ TileRange plan_tiles(int64_t n) {
-    const int64_t tiles = (n + kPlanThreads - 1) / kPlanThreads;
-    return TileRange{tiles * blockIdx.x / gridDim.x, tiles * (blockIdx.x + 1) / gridDim.x};
+// Weight of the strings before string i: their number, and their items' by bytes. (Offsets that are
+// out of order give any weights; the shares partition the strings all the same.)
+__device__ __forceinline__ uint64_t plan_weight(const int64_t *offsets, int64_t i, int64_t total_bytes, int64_t multi_n,
+                                                int32_t seg_len) {
+    const int64_t d = multi_n > 0 ? i / multi_n : 0, at = offsets[i - d * multi_n];
+    return (uint64_t)i + (uint64_t)(d * total_bytes + min(max(at, (int64_t)0), total_bytes)) / (uint32_t)seg_len;
+}
+__device__ __forceinline__ StringRange plan_strings(const int64_t *offsets, int64_t n, int64_t total_bytes, int32_t seg_len,
+                                                    int64_t multi_n, int n_dfas) {
+    const int64_t G = gridDim.x, c = blockIdx.x, tiles = (n + kPlanThreads - 1) / kPlanThreads;
+    // a few tiles a CTA: equal numbers of tiles, which a share by weight would cut through
+    if (tiles <= 4 * G) return StringRange{tiles * c / G * kPlanThreads, min(n, tiles * (c + 1) / G * kPlanThreads)};
+    // Weights at kPlanThreads evenly spaced strings; a border lies where its part of the total falls
+    // between two of them. The number of weights below a bound grows with the bound, so the borders
+    // are in order whatever the weights are.
+    __shared__ uint64_t s_weight[kPlanThreads + 1];
+    const int64_t t = threadIdx.x;
+    const uint64_t mine = plan_weight(offsets, n * t / kPlanThreads, total_bytes, multi_n, seg_len);
+    const uint64_t all = (uint64_t)n + (uint64_t)(total_bytes * (multi_n > 0 ? n_dfas : 1)) / (uint32_t)seg_len;
+    s_weight[t] = mine;
+    if (t == 0) s_weight[kPlanThreads] = all;
+    __syncthreads();
+    auto border = [&](int64_t k) -> int64_t {
+        const double bound = (double)all * ((double)k / (double)G);
+        const int below = __syncthreads_count((double)mine < bound);
+        if (k == 0 || k == G) return k == 0 ? 0 : n;
+        if (below == 0) return 0;
+        const double w0 = (double)s_weight[below - 1], w1 = (double)s_weight[below];
+        const int64_t x0 = n * (below - 1) / kPlanThreads, x1 = n * below / kPlanThreads;
+        return bound <= w0 ? x0 : bound >= w1 ? x1 : min(x1, x0 + (int64_t)((double)(x1 - x0) * ((bound - w0) / (w1 - w0))));
+    };
+    const int64_t first = border(c);
+    return StringRange{first, border(c + 1)};
 }
 
 // Counts the items of every (DFA, length class) and the map slots of this CTA's
@@ -325,13 +355,10 @@ plan_count_kernel(const int64_t *offsets, const int32_t *dfa_id, int64_t n, int6
     for (int t = threadIdx.x; t < n_bins; t += blockDim.x) cnt[t] = 0;
     if (threadIdx.x == 0) { items = 0; maps = 0; splits = 0; }
     __syncthreads();
-    const TileRange range = plan_tiles(n);
-    StringIn cur = range.first < range.end
-                       ? load_string(offsets, dfa_id, range.first * kPlanThreads + threadIdx.x, n, multi_n)
-                       : StringIn{0, 0, 0, false};
-    for (int64_t tile = range.first; tile < range.end; ++tile) {
-        const StringIn nxt =
-            load_string(offsets, dfa_id, (tile + 1) * kPlanThreads + threadIdx.x, n, multi_n);
+    const StringRange mine = plan_strings(offsets, n, total_bytes, seg_len, multi_n, n_dfas);
+    StringIn cur = load_string(offsets, dfa_id, mine.first + threadIdx.x, mine.end, multi_n);
+    for (int64_t at = mine.first; at < mine.end; at += kPlanThreads) {
+        const StringIn nxt = load_string(offsets, dfa_id, at + kPlanThreads + threadIdx.x, mine.end, multi_n);
         int64_t len = 0, s0 = 0;
         const int d = checked_loaded(cur, n_dfas, total_bytes, err, &len, &s0);
         cur = nxt;
@@ -525,14 +552,11 @@ plan_fill_kernel(const int64_t *offsets, const int32_t *dfa_id, int64_t n, int64
     }
     __syncthreads();
     bool bad = false;
-    const TileRange range = plan_tiles(n);
-    StringIn cur = range.first < range.end
-                       ? load_string(offsets, dfa_id, range.first * kPlanThreads + threadIdx.x, n, multi_n)
-                       : StringIn{0, 0, 0, false};
-    for (int64_t tile = range.first; tile < range.end; ++tile) {
-        const int64_t i = tile * kPlanThreads + threadIdx.x;
-        const StringIn nxt =
-            load_string(offsets, dfa_id, (tile + 1) * kPlanThreads + threadIdx.x, n, multi_n);
+    const StringRange mine = plan_strings(offsets, n, total_bytes, seg_len, multi_n, n_dfas);
+    StringIn cur = load_string(offsets, dfa_id, mine.first + threadIdx.x, mine.end, multi_n);
+    for (int64_t at = mine.first; at < mine.end; at += kPlanThreads) {
+        const int64_t i = at + threadIdx.x;
+        const StringIn nxt = load_string(offsets, dfa_id, at + kPlanThreads + threadIdx.x, mine.end, multi_n);
         int64_t len = 0, s0 = 0;
         const int d = checked_loaded(cur, n_dfas, total_bytes, err, &len, &s0);
         cur = nxt;
