@@ -93,3 +93,25 @@ def test_strings_cut_into_units(cuda, oracle, kind, shape, n):
     if rejects:
         data[rng.integers(0, data.size, size=3)] = sigma + 1
     _check(cuda, oracle, T, start, acc, data, off, rejects)
+
+
+def test_cut_string_past_four_billion(cuda, oracle):
+    # a cut string whose index needs more than 32 bits (its units are found by that index)
+    from trex_b200.engine import NFA
+    if cuda.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 75 GB of device memory")
+    rng = np.random.default_rng(9)
+    T, start, acc = random_bool_nfa(rng, 64, 20, density=0.05)
+    n, L = (1 << 32) + 3, 200003
+    data = rng.integers(0, 20, size=L, dtype=np.uint8)
+    off = cuda.zeros(n + 1, dtype=cuda.int64, device="cuda")
+    off[-2:] = L                                   # string 2^32 + 1; the one after it is empty
+    m = NFA(T, start, acc, unknown_rejects=False)
+    mask, ok = m.run(cuda.from_numpy(data).cuda(), off)
+    assert m.error_word() == 0
+    want, wacc = oracle.nfa_bool(T, start, acc, data, np.array([0, L, L]), unknown_rejects=False)
+    m.close()
+    for i, k in ((n - 2, 0), (n - 1, 1), (0, 1), (1, 1), (n - 3, 1)):
+        assert int(mask[i].item()) & (1 << 64) - 1 == int(np.uint64(want[k])) and int(ok[i].item()) == int(wacc[k])
+    del off, mask, ok
+    cuda.cuda.empty_cache()

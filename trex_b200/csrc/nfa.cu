@@ -34,10 +34,11 @@
 // and reports; the last reporter of a string whose guesses all hold writes the
 // last unit's set. Where a guess fails, the string is walked again from there
 // by one thread (for unit 0, whose set is always the true one, by its own
-// thread at once, so that an automaton whose guesses never hold takes no longer
-// than uncut), which jumps to a unit's end when it meets the unit's guess or its
+// thread at once), which jumps to a unit's end when it meets the unit's guess or its
 // checkpoint. Nobody waits for anybody. Exact for every NFA. 2048 log-normal
-// strings (median 2 KiB, longest 64 KiB), 64 states, 20 symbols: 7.7 -> 0.17 ms.
+// strings (median 2 KiB, longest 64 KiB), 64 states, 20 symbols: 7.7 -> 0.17 ms. An automaton whose
+// guesses never hold (permutations) pays for the looks at every unit: one string of 64 KiB, 10 / 20 /
+// 60 symbols, 3.39 / 3.61 / 4.88 ms, uncut 3.09 / 3.30 / 4.66; 2000 strings of 4 KiB 0.34 ms, uncut 2.7.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -98,7 +99,8 @@ constexpr int kNfaUnitsPerSm = 64;
 enum : uint32_t { kUnitGuess = 1u, kUnitDone = 2u, kUnitBroken = 4u };   // Broken: the next guess fails
 struct NfaUnit {
     uint64_t guess, exit, check;   // sets at the cut, at the end, at the checkpoint
-    uint32_t str, word;            // string; index << 8 | flags
+    int64_t str;
+    uint32_t word;                 // index << 8 | flags
     // unit 0 has no guess: the string's reports (low half) and failed guesses
     __device__ uint32_t *reports() { return reinterpret_cast<uint32_t *>(&guess); }
     __device__ uint32_t *broken() { return reinterpret_cast<uint32_t *>(&guess) + 1; }
@@ -138,7 +140,7 @@ __global__ void nfa_units_kernel(NfaParams P, uint32_t *n_units) {
             at = __shfl_sync(FULL, at, 0);
             if (at > P.max_units || at + ks > P.max_units) continue;
             for (uint32_t j = lane; j < ks; j += 32u)
-                P.units[at + j] = NfaUnit{0, 0, 0, (uint32_t)(base + l), j << 8};
+                P.units[at + j] = NfaUnit{0, 0, 0, base + l, j << 8};
         }
     }
 }
@@ -227,7 +229,7 @@ __device__ __forceinline__ void nfa_walk_units(const NfaParams &P, const typenam
         const unsigned long long q = atomicAdd(P.head, 1ull);
         if (q >= (unsigned long long)P.n + U) break;
         NfaUnit *u = q < U ? P.units + q : nullptr;   // the unit walked
-        const int64_t i = u ? (int64_t)u->str : (int64_t)q - U;
+        const int64_t i = u ? u->str : (int64_t)q - U;
         const int64_t a = P.offsets[i], b = P.offsets[i + 1];
         if (a < 0 || b < a || b > P.total_bytes) {
             if (!u) atomicOr(P.err, 1u);
