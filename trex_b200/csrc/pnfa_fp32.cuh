@@ -207,6 +207,11 @@ __device__ __noinline__ void ri_feed(const RiParams &P) {
     if (lane < cnt) {
         ri_fence();
         ri_st16(ri_entry(P, (uint32_t)P.n_rings, head + lane), kRiNone);
+    }
+    // every place is free before a slot goes on: its string can end and come back to one of them
+    // (with as many slots as places)
+    __syncwarp();
+    if (lane < cnt) {
         const uint4 w = ri_ld128(ri_base() + P.recs_off + slot * kRiRecBytes + kRiRecE);
         const double dot = (double)__uint_as_float(w.w);
         const int64_t E = (int64_t)(((uint64_t)w.y << 32) | w.x);
