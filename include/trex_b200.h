@@ -170,9 +170,12 @@ int64_t trex_dfa_batch_scratch_bytes(int64_t n_strings, int64_t total_bytes, int
  * final_state[n], accept[n] (uint8 0/1), accept_i32[n] (int 0/1).
  * scratch: at least trex_dfa_batch_scratch_bytes bytes, 16-byte aligned (as
  * cudaMalloc returns; else TREX_ERR_ARG), or NULL to use a buffer owned by the
- * set. seg_len: characters per work item (0 = default;
- * longer strings are split and their segment maps composed). stream: a
- * cudaStream_t (NULL = legacy default stream). */
+ * set. seg_len: characters per work item (longer strings are split and their
+ * items chained; 0 = default). At 0 a batch of at most 8 MiB walked and 131072
+ * strings, on a set with at most 200 KiB of byte maps, runs in one launch that
+ * plans no items and walks bytes, whatever trex_dfa_set_kgram has set; an explicit
+ * length always plans. Results are the same. stream: a cudaStream_t (NULL =
+ * legacy default stream). */
 int trex_dfa_batch_run(trex_dfa_set *set, const uint8_t *data, const int64_t *offsets,
                        const int32_t *dfa_id, int64_t n_strings, int64_t total_bytes,
                        uint8_t *final_state, uint8_t *accept, int32_t *accept_i32,

@@ -30,6 +30,45 @@ def test_cache_file_round_trip(tmp_path):
     assert Autotuner(cache_path=str(p)).cache == t.cache
 
 
+class _FakeSet:
+    """Records the item length of every run and how wide the grams were."""
+
+    def __init__(self, dfas):
+        self.dfas, self.k, self.runs = dfas, [1] * len(dfas), []
+
+    def kgram_max(self, d):
+        return 4
+
+    def set_kgram(self, d, k):
+        self.k[d] = k
+
+    def run(self, data, offsets, ids, seg_len=0):
+        self.runs.append((seg_len, tuple(self.k)))
+
+
+def test_gram_widths_are_timed_on_planned_items_and_the_default_is_a_candidate(tmp_path):
+    import torch
+    from types import SimpleNamespace
+    rng = np.random.default_rng(1)
+    off = np.arange(0, 101, dtype=np.int64) * 30   # a small batch: the default length walks bytes
+    data = torch.from_numpy(rng.integers(0, 256, size=3000, dtype=np.uint8))
+    t = Autotuner(cache_path=str(tmp_path / "t.json"))
+    # the widest gram and the library's default are the fastest
+    t._time = lambda fn: (fn(), 10 - s.runs[-1][1][0] + (s.runs[-1][0] > 0))[1]
+    s = _FakeSet([SimpleNamespace(n_states=16)])
+    rep = t.tune_batch(s, data, off)
+    gram_runs = s.runs[:3]
+    assert [k for _, (k,) in gram_runs] == [1, 2, 4] and all(seg > 0 for seg, _ in gram_runs)
+    assert rep.kgram == [4] and rep.seg_len == 0
+    assert sorted(seg for seg, _ in s.runs[3:]) == sorted(SEG_CANDIDATES) and 0 in SEG_CANDIDATES
+    # a batch of as many strings but many more bytes is not tuned by this one
+    wide = np.concatenate([off[:-1], [off[-1] + 400000]])
+    big = torch.zeros(int(wide[-1]), dtype=torch.uint8)
+    runs = len(s.runs)
+    rep2 = t.tune_batch(s, big, wide)
+    assert not rep2.cached and len(s.runs) > runs
+
+
 @pytest.mark.gpu
 def test_tuned_batch_matches_oracle_and_caches(cuda, oracle, tmp_path):
     from trex_b200.engine import DFASet

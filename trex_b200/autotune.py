@@ -7,7 +7,9 @@ measured on the GPU on a sample of the caller's own batch:
 * K-gram width, per automaton: every width the automaton allows
   (``DFASet.kgram_max``: 1, 2, 4, 8) is timed on the automaton's own strings;
 * tile shape of the ragged kernel (bytes per work item, ``seg_len``), per batch:
-  a sweep over 512 .. 8192 bytes with the chosen widths;
+  a sweep over 512 .. 8192 bytes with the chosen widths, and 0, the library's
+  default: small batches then run in one launch that plans no items and walks
+  bytes (K-gram widths are timed with an explicit length, which plans);
 * scan block size (bytes per scan tile, ``tile_len``) of the per-position
   scan, per automaton and string length, measured on the whole batch (up to
   ``scan_bytes``): the scan's parallelism comes from the tiles of all strings
@@ -18,12 +20,12 @@ Each candidate is timed with CUDA events around the library call (median of
 are cached in a JSON file keyed by automaton size and shape of the input, so a
 second batch of the same kind is not measured again:
 
-    dfa:N<=8|16|256:k<=K:len<L       -> K-gram width
-    seg:d<D:n<S:len<L:k<K            -> bytes per work item
+    gram:N<=8|16|256:k<=K:len<L      -> K-gram width
+    seg:d<D:n<S:len<L:bytes<B:k<K    -> bytes per work item (0: the library default)
     scan:N<=8|16:n<S:len<L           -> scan tile length (0: the library default)
 
-(``len<L``: median string length rounded up to a power of two; ``n<S``:
-number of strings, likewise.) The cache path is ``cache_path``, else the
+(``len<L``: median string length rounded up to a power of two; ``n<S``,
+``bytes<B``: number of strings and of bytes, likewise.) The cache path is ``cache_path``, else the
 environment variable ``TREX_TUNE_CACHE``, else no file (in-memory only).
 """
 
@@ -38,7 +40,8 @@ from typing import Optional
 
 import numpy as np
 
-SEG_CANDIDATES = (512, 1024, 2048, 4096, 8192)
+SEG_CANDIDATES = (0, 512, 1024, 2048, 4096, 8192)   # 0: the library's default for the batch
+GRAM_SEG = 2048   # item length of the K-gram timings: at the default a small batch is walked by bytes
 SCAN_CANDIDATES = (0, 1024, 4096, 16384, 65536)   # 0: the library's default for the batch
 
 
@@ -159,7 +162,7 @@ class Autotuner:
             rows = np.flatnonzero(ids == d)
             med = _pow2_ceil(np.median(lens[rows])) if rows.size else 1
             N = dfa_set.dfas[d].n_states
-            key = f"dfa:N<={_n_class(N)}:k<={kmax}:len<{med}"
+            key = f"gram:N<={_n_class(N)}:k<={kmax}:len<{med}"
             if kmax == 1 or rows.size == 0:
                 k = 1
             elif key in self.cache:
@@ -174,7 +177,7 @@ class Autotuner:
                     if kk > kmax:
                         break
                     dfa_set.set_kgram(d, kk)
-                    ms = self._time(lambda: dfa_set.run(sdata, soff, sub_ids))
+                    ms = self._time(lambda: dfa_set.run(sdata, soff, sub_ids, seg_len=GRAM_SEG))
                     rep.sweep.append({"what": f"kgram[{d}]", "value": kk, "ms": ms,
                                       "bytes": int(soff[-1].item())})
                     if best is None or ms < best[1]:
@@ -188,7 +191,8 @@ class Autotuner:
                 dfa_set.set_kgram(d, 1)
         # work-item length for the whole batch, with the chosen widths
         med = _pow2_ceil(np.median(lens)) if lens.size else 1
-        key = f"seg:d<{_pow2_ceil(n_dfas)}:n<{_pow2_ceil(len(lens))}:len<{med}:k<{max(rep.kgram or [1])}"
+        key = (f"seg:d<{_pow2_ceil(n_dfas)}:n<{_pow2_ceil(len(lens))}:len<{med}:bytes<{_pow2_ceil(int(off[-1]))}"
+               f":k<{max(rep.kgram or [1])}")
         if key in self.cache:
             rep.seg_len = int(self.cache[key])
         else:
