@@ -298,8 +298,16 @@ class DFAWorkload:
         return self.total
 
     @property
+    def one_launch(self):
+        # small batches at the default item length (see trex_dfa_batch_run in include/trex_b200.h)
+        return (self.kind != "scan" and not self.args.seg_len and self.n <= 131072 and self.total <= 8 << 20
+                and sum(256 * d.n_states for d in self.dfas) <= 200 << 10)
+
+    @property
     def kernel(self):
-        return "dfa_scan_kernel" if self.kind == "scan" else "dfa_ragged_kernel"
+        if self.kind == "scan":
+            return "dfa_scan_kernel"
+        return "dfa_small_kernel" if self.one_launch else "dfa_ragged_kernel"
 
     @property
     def alg_bytes(self):
@@ -310,13 +318,13 @@ class DFAWorkload:
 
     @property
     def launches_per_step(self):
-        # scan: tile bases, empty strings, scan; ragged: count, class prefix, queue scan, fill,
-        # walk, and chaining (records, fix-ups, re-walks)
-        return 3 if self.kind == "scan" else 8
+        # scan: plan, scan; ragged: count, class prefix, queue scan, fill, walk, and chaining
+        # (records, fix-ups, re-walks); a small batch one kernel
+        return 2 if self.kind == "scan" else 1 if self.one_launch else 8
 
     def config(self):
         return {"workload": self.workload, "n_strings": self.n, "total_bytes_per_gpu": self.total,
-                "seg_len": self.args.seg_len or (8192 if self.kind == "scan" else 2048),
+                "seg_len": self.args.seg_len or (8192 if self.kind == "scan" else 0 if self.one_launch else 2048),
                 "kgram": getattr(self, "kgram_used", None),
                 "l2": "inputs larger than L2 (126 MB), no flush" if self.total > 126e6 else
                       "inputs smaller than L2: L2 flushed by a 256 MB write between steps"}
@@ -414,7 +422,7 @@ class NFAWorkload:
 
     kind = "nfa"
     kernel = "nfa_bitpar_kernel"
-    launches_per_step = 1
+    launches_per_step = 2   # units of cut strings, walk
     dtype = ref_dtype = "u64"
 
     def __init__(self, args):

@@ -483,6 +483,7 @@ int nfa_run(trex_nfa *nfa, const uint8_t *data, const int64_t *offsets, int64_t 
     P.max_units = nfa->max_units;
     P.seg = std::max(kNfaMinSeg, (total_bytes / ((int64_t)nfa->n_sms * kNfaUnitsPerSm) + 15) & ~(int64_t)15);
     P.all_states = nfa->n_states == 64 ? ~0ull : (1ull << nfa->n_states) - 1;
+    profile_kernel_begin(stream);   // (the listing kernel is part of the run)
     if (total_bytes > P.seg) {
         const int ugrid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)nfa->n_sms);
         nfa_units_kernel<<<ugrid, 256, 0, stream>>>(P, err + 1);
@@ -493,7 +494,6 @@ int nfa_run(trex_nfa *nfa, const uint8_t *data, const int64_t *offsets, int64_t 
     // automata launched on separate streams run side by side
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(nfa->n_sms, std::max((n + 31) / 32, total_bytes / (32 * P.seg))));
-    profile_kernel_begin(stream);
     nfa->lay->run<<<grid, kNfaThreads, smem, stream>>>(P);
     TREX_CHECK_LAUNCH();
     profile_kernel_end(stream);
