@@ -40,7 +40,8 @@ position), dfa_n32_64 (the ragged batch shape, 250K strings, on 32- and
 gram tables apply), ref_shapes (the NFA kernels on the shape the reference
 publishes its NFA numbers for: sigma 2, 262144 x 2048, with those numbers
 beside them), cfg5_served (a Poisson sweep up to saturation, with the limiter
-named). --no-extras skips them.
+named). --no-extras skips them. The line on stdout holds their values only; the full
+record, with sweeps, verification and rooflines, goes to stderr.
 
 Multi-GPU: one process per GPU (torchrun); every rank runs its own seeded
 batch (weak scaling, no data-path collective); times are the max over ranks
@@ -1571,6 +1572,29 @@ def ref_shapes(args, torch, dev):
     return {"shape": f"64-state NFAs over 2 symbols, {R} strings x 2048 symbols", "by_kernel": out}
 
 
+def short_line(line):
+    """The line for stdout: the headline's keys with the kernel's roofline, and of every other
+    workload its value, few enough characters that whoever keeps the end of the output has all of
+    it. The full record goes to stderr."""
+    def brief(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        if isinstance(v, dict):
+            return {k: brief(x) for k, x in v.items()}
+        return [brief(x) for x in v] if isinstance(v, list) else v
+    out = {k: v for k, v in line.items() if k not in ("autotune", "cpu_baseline", "configs", "roofline")}
+    out["config"] = {k: v for k, v in line["config"].items() if k not in ("kgram", "total_bytes_per_gpu")}
+    if "mismatches_vs_oracle" in out and isinstance(out["mismatches_vs_oracle"], dict):
+        out["mismatches_vs_oracle"] = {k: v for k, v in out["mismatches_vs_oracle"].items() if k not in ("strings", "bytes")}
+    out["roofline"] = {k: line["roofline"][k] for k in ("bound", "frac", "kernel", "kernel_ms_mean")}
+    if line.get("cpu_baseline"):
+        out["cpu_baseline"] = {k: line["cpu_baseline"][k] for k in ("value", "cores", "kind")}
+    if "configs" in line:
+        out["configs"] = {k: float(f"{v['value']:.4g}") for k, v in line["configs"].items()
+                          if isinstance(v, dict) and isinstance(v.get("value"), (int, float))}
+    return brief(out)
+
+
 def trex_arm(args, rank, world, local_rank):
     import torch
     dev = torch.device("cuda", local_rank)
@@ -1607,7 +1631,8 @@ def trex_arm(args, rank, world, local_rank):
                 failed |= isinstance(v, dict) and failed_checks(v)
         else:
             wl.close()
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(line)), flush=True)
     else:
         wl.close()
     if failed:
