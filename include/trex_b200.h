@@ -46,9 +46,11 @@ const char *trex_version(void);
  * look-back spins without a limit, cuda/monoid_scan.cu:187-193): scan_polls =
  * polls of one look-back step of trex_dfa_scan_run, mbar_cycles = clock cycles
  * of one hand-off inside the NFA kernels (trex_pnfa_run modes BF16, FP16, BOOL,
- * BOOL8, FP32). A wait that runs out sets the timeout bit (4) of
- * the run's error word and the kernel returns; the results of that run are
- * then invalid. 0 restores a default (2^24 polls; 4e9 cycles, about 2 s).
+ * BOOL8, FP32): a wait for products or for work is given up when it runs out; a
+ * meeting of a CTA's warps at a hardware barrier (more than four symbols, 16-bit
+ * and Boolean modes) is timed, and the run ends after one that took longer.
+ * Either sets the timeout bit (4) of the run's error word and the kernel returns;
+ * the results of that run are then invalid. 0 restores a default (2^24 polls; 4e9 cycles, about 2 s).
  * Process-wide, read at each launch; meant for tests of the give-up paths. */
 int trex_set_wait_limits(int64_t scan_polls, int64_t mbar_cycles);
 

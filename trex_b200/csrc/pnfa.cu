@@ -21,7 +21,9 @@
 // table in each warp's registers and bring the strings to it (mma.sync, pnfa_sym.cuh). FP32:
 // tables on the SM (pnfa_fp32.cuh), or through L1 for alphabets that do not fit. The
 // low-latency forms with 16-bit tables are at the end.
-// Every wait is bounded; one that runs out sets the error word (bit 2).
+// A wait at an mbarrier or a ring is bounded, a meeting at a hardware barrier is timed afterwards
+// (its warps never wait for another CTA); one that ran out or took too long sets the error word
+// (bit 2) and ends the run.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -40,7 +42,7 @@ constexpr uint32_t kPnSmemCap = 232448;
 constexpr uint32_t kPnErrOffsets = 1u, kPnErrTimeout = 4u;
 // The drain of committed MMAs before the TMEM is freed always waits up to the
 // default limit (an MMA still writing TMEM must not outlive the allocation);
-// the hand-off waits use PnParams::wait_cycles.
+// the hand-off waits use the run's own limit.
 constexpr long long kPnDrainCycles = kDefaultMbarCycles;
 
 __host__ __device__ inline uint32_t pn_align16(uint32_t x) { return (x + 15u) & ~15u; }
@@ -66,13 +68,24 @@ __device__ __forceinline__ bool pn_mbar_test(uint32_t addr, uint32_t parity) {
         : "=r"(done) : "r"(addr), "r"(parity) : "memory");
     return done != 0;
 }
+// The same without the pause that the hardware may take before it answers.
+__device__ __forceinline__ bool pn_mbar_look(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    return done != 0;
+}
 // The warp waits for the completion of the phase with the given parity; bounded, the same result
-// in all lanes. A thread whose phase is not complete may be parked by the hardware (try_wait).
+// in all lanes. A limit shorter than the hardware's pause starts with a look, so that it holds (the
+// look costs a tile of a few int8 strings up to a tenth of its time).
 __device__ __forceinline__ bool ln_wait(uint32_t addr, uint32_t parity, volatile uint32_t *abort_flag,
                                         uint32_t *err, long long limit) {
     bool ok = true;
     const long long t0 = clock64();
-    while (!pn_mbar_test(addr, parity)) {
+    for (bool done = limit < 1000 ? pn_mbar_look(addr, parity) : pn_mbar_test(addr, parity); !done;
+         done = pn_mbar_test(addr, parity)) {
         if (*abort_flag) { ok = false; break; }
         if (clock64() - t0 > limit) {
             atomicOr(err, kPnErrTimeout);
@@ -141,15 +154,12 @@ __device__ __forceinline__ void pn_tmem_st16(uint32_t taddr, const uint32_t (&r)
 // writes its next A row with tcgen05.st; at the string's end it forms the log-likelihood and
 // takes the next string from the queue.
 //
-// Bound by the latency of a tile's step (the 512 TMEM columns hold no more strings): 4900 cycles
-// before, alike with one tile and with four, now about half. 262144 strings x 2048 symbols, 2 symbols,
-// FP16: 20.27 -> 10.70 ms; x 512 symbols, ms before / now, for 2, 3, 4 symbols: BF16 4.58 / 2.46,
-// 5.88 / 3.12, 8.37 / 4.26; FP16 5.14 / 2.85, 6.49 / 3.41, 9.14 / 4.65; int8 4.87 / 2.15, 4.98 / 2.29,
-// 5.15 / 2.53. Before, warps of their own waited at an mbarrier for the tile, read its liveness
-// from shared memory and issued the products, and the next symbol was found after them.
-// So a step has one hand-off: the four warps of a tile meet at a hardware barrier, which also
-// tells whether any string is left, an elected thread of the first issues the products, and the
-// next symbol is found while they run; a tcgen05.commit brings the result (a bounded wait).
+// Bound by the latency of a tile's step, about 2500 cycles (the 512 TMEM columns hold no more
+// strings): 262144 strings x 2048 symbols, 2 symbols, FP16 take 10.70 ms (20.27 with a warp of its
+// own to issue the products, and two hand-offs a step). A step has one hand-off: the four warps of
+// a tile meet at a hardware barrier, which also tells whether any string is left, an elected thread
+// of the first issues the products, and the next symbol is found while they run; a tcgen05.commit
+// brings the result (a bounded wait).
 constexpr int kLnTiles = 4;
 constexpr int kLnEpiWarps = 4 * kLnTiles;   // tile T: warps 4T .. 4T + 3 (lane quadrants 0-3)
 constexpr int kLnThreads = 32 * kLnEpiWarps;
@@ -450,7 +460,7 @@ __global__ void __launch_bounds__(kLnThreads, 1) pnfa_lane_kernel(const __grid_c
             if (qd == 0) {
                 // One K chain (4 sigma K16 or 2 sigma K32 steps), issued by an elected thread with
                 // the steps unrolled: 37-43 cycles an MMA (M = 128, N = 64, K = 16 takes 32); a loop
-                // under `lane == 0` moves every operand to a uniform register: 103-109.
+                // under `lane == 0` took 103-109.
                 if (ln_elect()) {
                     // K step kk: B 2 kLnLbo bytes further (+128 in the descriptor's start field,
                     // which stays below 2^14 for shared addresses), A 8 TMEM columns further
