@@ -157,8 +157,8 @@ __device__ inline void build_layout(int N, int ncols, uint32_t off, F next) {
 // four states of one byte and is the same in every replica (but for the lane bits of the smallest
 // layout), so a warp forms 32 different words, one a lane, and then writes each one's replicas
 // together. Bound by the byte loads of the map: a word's four are made once and not once a replica
-// (100K strings on 32- and 64-state automata: 409 -> 400 us a batch; ragged scan of 3001 strings:
-// 121 -> 116 us; 1M strings on 16 automata: 1328 -> 1314 us). Not inlined: the walkers keep their registers.
+// (ragged scan of 3001 strings: 121 -> 116 us; 1M strings on 16 automata: 1336 -> 1332 us). Not inlined:
+// the walkers keep their registers.
 static __device__ __noinline__ void build_table(const uint8_t *__restrict__ src, int N) {
     if (N <= 64) {
         // words of a byte's column: ceil(states / 4) rounded to the layout; bits a state group

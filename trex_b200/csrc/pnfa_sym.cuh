@@ -18,10 +18,7 @@
 // append) with five warps a scheduler to hide it: 65536 strings x 2048 symbols, 20 symbols, BF16
 // take 7.03 ms, of which the MMAs' issue (2 cycles each on an SM) is 1.9 ms. tcgen05.mma needs 128
 // rows of A, two symbols' tables, throws half of every product away and brings it back through
-// TMEM: that form, with a step's strings sorted by symbol pair, took 20.65 ms here (at 512
-// symbols, Gchar/s, that form / this one: BF16 6.4 / 18.5, FP16 5.5 / 14.7, Boolean int8 7.3 /
-// 24.4, Boolean BF16 7.0 / 18.2; 2000 strings 3.57 / 0.59 ms, 100 strings x 2048 symbols 14.0 /
-// 1.67 ms). With mbarriers between the warps of a symbol instead of one barrier a step it took
+// TMEM: that form, with a step's strings sorted by symbol pair, took 20.65 ms. With mbarriers between the warps of a symbol instead of one barrier a step it took
 // 12.1 ms: a warp that polls takes issue slots and the shared-memory pipe from those that work.
 #pragma once
 
@@ -30,7 +27,7 @@ namespace trex {
 constexpr int kSyWarps = 20;            // 5 a scheduler: 96 registers a thread
 constexpr int kSyThreads = 32 * kSyWarps;
 constexpr int kSyMaxSigma = 28;
-constexpr int kSyMaxSlots = 512;        // a thread a slot
+constexpr int kSyMaxSlots = 512;        // a thread keeps one or two (11 to 15 symbols launch fewer threads)
 constexpr int kSyBlk = 16;              // steps a block
 constexpr uint32_t kSyEnd = 0xFFu;      // symbol after a string's last
 // a slot: free, walking a string, or its string ended and the result is to be written
