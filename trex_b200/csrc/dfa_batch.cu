@@ -309,7 +309,7 @@ struct StringRange {
 // out of order give any weights; the shares partition the strings all the same.)
 __device__ __forceinline__ uint64_t plan_weight(const int64_t *offsets, int64_t i, int64_t total_bytes, int64_t multi_n,
                                                 int32_t seg_len) {
-    const int64_t d = multi_n > 0 ? i / multi_n : 0, at = offsets[i - d * multi_n];
+    const int64_t d = multi_n > 0 ? (uint32_t)i / (uint32_t)multi_n : 0, at = offsets[i - d * multi_n];   // (below 2^31 strings)
     return (uint64_t)i + (uint64_t)(d * total_bytes + min(max(at, (int64_t)0), total_bytes)) / (uint32_t)seg_len;
 }
 __device__ __forceinline__ StringRange plan_strings(const int64_t *offsets, int64_t n, int64_t total_bytes, int32_t seg_len,

@@ -99,8 +99,9 @@ constexpr int kNfaUnitsPerSm = 64;
 enum : uint32_t { kUnitGuess = 1u, kUnitDone = 2u, kUnitBroken = 4u };   // Broken: the next guess fails
 struct NfaUnit {
     uint64_t guess, exit, check;   // sets at the cut, at the end, at the checkpoint
-    int64_t str;
-    uint32_t word;                 // index << 8 | flags
+    uint32_t str, word;            // string, low half; its next 8 bits << 24 | index << 8 | flags
+    __device__ int64_t string() const { return (int64_t)(((uint64_t)(word >> 24) << 32) | str); }
+    __device__ uint32_t index() const { return (word >> 8) & 0xFFFFu; }
     // unit 0 has no guess: the string's reports (low half) and failed guesses
     __device__ uint32_t *reports() { return reinterpret_cast<uint32_t *>(&guess); }
     __device__ uint32_t *broken() { return reinterpret_cast<uint32_t *>(&guess) + 1; }
@@ -140,7 +141,7 @@ __global__ void nfa_units_kernel(NfaParams P, uint32_t *n_units) {
             at = __shfl_sync(FULL, at, 0);
             if (at > P.max_units || at + ks > P.max_units) continue;
             for (uint32_t j = lane; j < ks; j += 32u)
-                P.units[at + j] = NfaUnit{0, 0, 0, base + l, j << 8};
+                P.units[at + j] = NfaUnit{0, 0, 0, (uint32_t)(base + l), (uint32_t)((uint64_t)(base + l) >> 32) << 24 | j << 8};
         }
     }
 }
@@ -229,7 +230,7 @@ __device__ __forceinline__ void nfa_walk_units(const NfaParams &P, const typenam
         const unsigned long long q = atomicAdd(P.head, 1ull);
         if (q >= (unsigned long long)P.n + U) break;
         NfaUnit *u = q < U ? P.units + q : nullptr;   // the unit walked
-        const int64_t i = u ? u->str : (int64_t)q - U;
+        const int64_t i = u ? u->string() : (int64_t)q - U;
         const int64_t a = P.offsets[i], b = P.offsets[i + 1];
         if (a < 0 || b < a || b > P.total_bytes) {
             if (!u) atomicOr(P.err, 1u);
@@ -238,7 +239,7 @@ __device__ __forceinline__ void nfa_walk_units(const NfaParams &P, const typenam
         const uint32_t k = U ? nfa_units_of(P.data, a, b, P.seg) : 1u;
         if (!u && k > 1u) continue;
         const int64_t c0 = nfa_cut0(P.data, a);
-        uint32_t j = u ? u->word >> 8 : 0u;
+        uint32_t j = u ? u->index() : 0u;
         NfaUnit *const u0 = u - j;
         auto cut = [&](uint32_t x) { return x == 0u ? a : x >= k ? b : c0 + (int64_t)x * P.seg; };
         // stage 0: the warm-up; 1: to the checkpoint; 2: to the unit's end
@@ -597,7 +598,7 @@ int trex_nfa_create(int n_states, int sigma, const uint64_t *cols, uint64_t star
         set_last_error_msg("trex_nfa_create: no CUDA device");
         return TREX_ERR_SHAPE;
     }
-    nfa->max_units = 2u * (uint32_t)nfa->n_sms * kNfaUnitsPerSm + 64u;
+    nfa->max_units = std::min(65535u, 2u * (uint32_t)nfa->n_sms * kNfaUnitsPerSm + 64u);   // (16-bit index)
     const size_t misc_off = (nfa->table_bytes + 255) & ~size_t(255);
     cudaError_t e;
     if ((e = cudaMalloc(&nfa->d_tables, misc_off + 256 + sizeof(NfaUnit) * nfa->max_units)) != cudaSuccess ||
