@@ -105,3 +105,22 @@ def test_fp32_long_skipped_runs_are_work(cuda, oracle):
     ref = oracle.pnfa_fp64(T, start, acc, data, off)
     assert np.all(np.abs(ll - ref) <= 1e-5 * np.abs(ref))   # at most 500 symbols, as above
     assert np.array_equal(ac.astype(bool), ref > np.log(0.5))
+
+
+# runs of skipped bytes around the words and lines that they are read by, at every alignment of the string
+@pytest.mark.parametrize("run", [1, 3, 4, 5, 63, 64, 65, 67, 127, 128, 131, 300])
+def test_fp32_skipped_runs_at_every_alignment(cuda, oracle, run):
+    rng = np.random.default_rng(run)
+    T, start, acc = (x.astype(np.float32) for x in random_prob_nfa(rng, 64, 7))
+    parts, off = [], [0]
+    for lead in range(70):
+        s = [np.full(lead % 3, 9), rng.integers(0, 7, size=lead), np.full(run, 200), rng.integers(0, 7, size=lead % 2),
+             np.full(run * (lead % 2), 255)]
+        parts.append(np.concatenate(s).astype(np.uint8))
+        off.append(off[-1] + len(parts[-1]))
+    data, off = np.concatenate(parts), np.array(off, dtype=np.int64)
+    ll, _, err = _run(cuda, T, start, acc, data, off)
+    ref = oracle.pnfa_fp64(T, start, acc, data, off)
+    fin = np.isfinite(ref)
+    assert err == 0 and np.array_equal(np.isfinite(ll), fin)
+    assert np.all(np.abs(ll - ref)[fin] <= 1e-6 + 1e-5 * np.abs(ref[fin]))   # at most 70 symbols, as above

@@ -135,23 +135,32 @@ __device__ __forceinline__ uint32_t ri_poll(const RiParams &P, uint32_t ring, ui
     return got == 0xffffffffu ? 32u : (uint32_t)__ffs(~got) - 1u;
 }
 
-// The first byte below sigma of [p, e), or e: 64 bytes a step, so that a long run of skipped
-// bytes does not take a round trip a byte. Every piece of 4 KiB counts as work done (ri_stalled).
+// The first byte below sigma of [p, e), or e: four bytes at a time to a 64-byte line, then a line a
+// step, so that a long run of skipped bytes does not take a round trip a byte. Every 4 KiB of a run
+// count as work done (ri_stalled).
 __device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_t *e, uint32_t sigma) {
     const uint32_t sig4 = sigma * 0x01010101u;
-    while (p < e && (reinterpret_cast<uintptr_t>(p) & 15u)) {
+    while (p < e && (reinterpret_cast<uintptr_t>(p) & 3u)) {
         if (__ldg(p) < sigma) return p;
         ++p;
     }
-    for (uint32_t steps = 1; e - p >= 64; p += 64, ++steps) {
-        uint32_t in = 0u;
+    while (e - p >= 4) {
+        if ((reinterpret_cast<uintptr_t>(p) & 63u) == 0u) {
+            for (uint32_t lines = 1; e - p >= 64; p += 64, ++lines) {
+                uint32_t in = 0u;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p) + k);
-            in |= __vcmpltu4(v.x, sig4) | __vcmpltu4(v.y, sig4) | __vcmpltu4(v.z, sig4) | __vcmpltu4(v.w, sig4);
+                for (int k = 0; k < 4; ++k) {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p) + k);
+                    in |= __vcmpltu4(v.x, sig4) | __vcmpltu4(v.y, sig4) | __vcmpltu4(v.z, sig4) | __vcmpltu4(v.w, sig4);
+                }
+                if (in) break;
+                if (lines % 64u == 0u) ri_add32(ri_base() + kRiSkips, 1u);
+            }
+            if (e - p < 4) break;
         }
-        if (in) break;
-        if (steps % 64u == 0u) ri_add32(ri_base() + kRiSkips, 1u);
+        const uint32_t in = __vcmpltu4(__ldg(reinterpret_cast<const uint32_t *>(p)), sig4);
+        if (in) return p + ((__ffs(in) - 1) >> 3);
+        p += 4;
     }
     while (p < e && __ldg(p) >= sigma) ++p;
     return p;
@@ -241,11 +250,11 @@ __device__ __forceinline__ bool ri_try_feed(const RiParams &P, uint32_t least) {
     return true;
 }
 
-// A wait without work: true when nothing moved in any ring, and no lane skipped on in its string,
-// for the limit of clock cycles (all lanes call it; mark and t0 carry over between calls).
-__device__ __forceinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
+// After a wait without work for the limit of clock cycles since t0: true when nothing moved in any ring,
+// and no lane skipped on in its string, since the last call (all lanes call it; mark and t0 carry
+// over between calls). Not inlined, as ri_next.
+__device__ __noinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
     const uint32_t lane = threadIdx.x & 31u;
-    if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) return false;
     const bool counts = (int)lane <= P.n_rings || lane == (kRiSkips - kRiTails) / 4u;
     const uint32_t v = counts ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
     const uint32_t sum = __reduce_add_sync(0xffffffffu, v);
@@ -265,6 +274,7 @@ __device__ __forceinline__ uint32_t ri_wait(const RiParams &P, uint32_t ring, ui
         if (ri_ld32(ri_base() + kRiDone)) return 0u;
         if (ri_try_feed(P, 1u)) continue;
         if (t0 == 0) t0 = clock64();
+        if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) continue;
         if (ri_stalled(P, mark, t0)) {
             if ((threadIdx.x & 31u) == 0u) {
                 atomicOr(P.err, kPnErrTimeout);
@@ -372,9 +382,9 @@ __global__ void __launch_bounds__(kRiThreads, 1) pnfa_fp32_kernel(const __grid_c
         if (own) {   // the symbol after this one (bytes >= sigma are skipped)
             const uint8_t *p, *e;
             ri_ldp(rec + kRiRecP, p, e);
-            const bool found = p < e && nc < (uint32_t)P.sigma;
-            if (p < e) ri_stp(rec + kRiRecP, ++p);
-            if (!found) nc = p < e ? ri_next(rec, (uint32_t)P.sigma) : 255u;
+            p += p < e;
+            ri_stp(rec + kRiRecP, p);
+            if (nc >= (uint32_t)P.sigma && p < e) nc = ri_next(rec, (uint32_t)P.sigma);
             ending = nc >= (uint32_t)P.sigma;
         }
         const uint32_t ends = __ballot_sync(FULL, ending);
