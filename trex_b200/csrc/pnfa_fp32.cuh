@@ -14,8 +14,8 @@
 // the plain kernel's order, k = 0 .. 63, and the state is rescaled by the exponent of max |s'|
 // at every step, as there: the states are the same bits.
 //
-// 8192 strings x 512, 20 symbols: 16.7 -> 1.73 ms (0.26 -> 2.4 Gchar/s), the shared-memory pipe
-// 81% busy (80 wavefronts of table a group, 16 of states a string).
+// 8192 strings x 512, 20 symbols: 16.7 -> 1.72 ms (0.26 -> 2.4 Gchar/s), the shared-memory pipe
+// 82% busy (80 wavefronts of table a group, 16 of states a string).
 #pragma once
 
 namespace trex {
@@ -55,7 +55,7 @@ struct RiParams {
 // Shared memory: control words, rings (n_rings, then that of ended slots), records, state rows,
 // tables.
 constexpr uint32_t kRiTails = 0;                        // uint32 [kRiWarps + 1]
-constexpr uint32_t kRiSkips = 4 * (kRiWarps + 1);       // pieces of skipped bytes (ri_skip)
+constexpr uint32_t kRiBusy = 4 * (kRiWarps + 1);        // lanes that look for a string or skip its bytes
 constexpr uint32_t kRiEndHead = 128, kRiLock = 132, kRiLive = 136, kRiDone = 140;
 constexpr uint32_t kRiAcc = 144;                        // float [64]
 constexpr uint32_t kRiStart = kRiAcc + 256;             // uint4 [16]
@@ -136,8 +136,7 @@ __device__ __forceinline__ uint32_t ri_poll(const RiParams &P, uint32_t ring, ui
 }
 
 // The first byte below sigma of [p, e), or e: four bytes at a time to a 64-byte line, then a line a
-// step, so that a long run of skipped bytes does not take a round trip a byte. Every 4 KiB of a run
-// count as work done (ri_stalled).
+// step, so that a long run of skipped bytes does not take a round trip a byte.
 __device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_t *e, uint32_t sigma) {
     const uint32_t sig4 = sigma * 0x01010101u;
     while (p < e && (reinterpret_cast<uintptr_t>(p) & 3u)) {
@@ -146,7 +145,7 @@ __device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_
     }
     while (e - p >= 4) {
         if ((reinterpret_cast<uintptr_t>(p) & 63u) == 0u) {
-            for (uint32_t lines = 1; e - p >= 64; p += 64, ++lines) {
+            for (; e - p >= 64; p += 64) {
                 uint32_t in = 0u;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -154,7 +153,6 @@ __device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_
                     in |= __vcmpltu4(v.x, sig4) | __vcmpltu4(v.y, sig4) | __vcmpltu4(v.z, sig4) | __vcmpltu4(v.w, sig4);
                 }
                 if (in) break;
-                if (lines % 64u == 0u) ri_add32(ri_base() + kRiSkips, 1u);
             }
             if (e - p < 4) break;
         }
@@ -165,23 +163,15 @@ __device__ __forceinline__ const uint8_t *ri_skip(const uint8_t *p, const uint8_
     while (p < e && __ldg(p) >= sigma) ++p;
     return p;
 }
-// The next symbol of a slot's string (its record at rec), 255 at its end; moves the record on.
-// Not inlined: the tables stay in registers.
-__device__ __noinline__ uint32_t ri_next(uint32_t rec, uint32_t sigma) {
-    const uint8_t *p, *e;
-    ri_ldp(rec + kRiRecP, p, e);
-    p = ri_skip(p, e, sigma);
-    if (p == e) return 255u;
-    ri_stp(rec + kRiRecP, p + 1);
-    return __ldg(p);
-}
 
 // Gives a slot the next string of the batch: its record, its start row and its first ring.
 // Strings without symbols get their result at once; false when the batch has no more strings.
 __device__ __forceinline__ bool ri_refill(const RiParams &P, uint32_t slot) {
+    bool found = false;
+    ri_add32(ri_base() + kRiBusy, 1u);
     for (;;) {
         const unsigned long long idx = atomicAdd(P.queue, 1ull);
-        if (idx >= (unsigned long long)P.n) return false;
+        if (idx >= (unsigned long long)P.n) break;
         const int64_t p0 = P.offsets[idx], p1 = P.offsets[idx + 1];
         if (p0 < 0 || p1 < p0 || p1 > P.total_bytes) {
             atomicOr(P.err, kPnErrOffsets);
@@ -201,8 +191,11 @@ __device__ __forceinline__ bool ri_refill(const RiParams &P, uint32_t slot) {
         const uint32_t row = ri_base() + P.rows_off + slot * kRiRowBytes;
         for (uint32_t k = 0; k < kRiRowBytes - 16u; k += 16u) ri_st128(row + k, ri_ld128(ri_base() + kRiStart + k));
         ri_push(P, ri_ring_of(P, c, slot), slot);
-        return true;
+        found = true;
+        break;
     }
+    ri_add32(ri_base() + kRiBusy, 0xffffffffu);
+    return found;
 }
 
 // The ended slots, up to 32 at a time (the calling warp holds the lock): results, next strings.
@@ -250,15 +243,16 @@ __device__ __forceinline__ bool ri_try_feed(const RiParams &P, uint32_t least) {
     return true;
 }
 
-// After a wait without work for the limit of clock cycles since t0: true when nothing moved in any ring,
-// and no lane skipped on in its string, since the last call (all lanes call it; mark and t0 carry
-// over between calls). Not inlined, as ri_next.
-__device__ __noinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
+// A wait without work: true when nothing moved in any ring for the limit of clock cycles while no lane was
+// looking for a string or skipping bytes of one, which ends by itself (all lanes call it; mark and t0
+// carry over between calls).
+__device__ __forceinline__ bool ri_stalled(const RiParams &P, uint32_t &mark, long long &t0) {
     const uint32_t lane = threadIdx.x & 31u;
-    const bool counts = (int)lane <= P.n_rings || lane == (kRiSkips - kRiTails) / 4u;
-    const uint32_t v = counts ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
+    if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) return false;
+    const uint32_t v = (int)lane <= P.n_rings ? ri_ld32(ri_base() + kRiTails + 4u * lane) : 0u;
     const uint32_t sum = __reduce_add_sync(0xffffffffu, v);
-    if (sum == mark) return true;
+    const bool busy = __any_sync(0xffffffffu, ri_ld32(ri_base() + kRiBusy) != 0u);
+    if (sum == mark && !busy) return true;
     mark = sum;
     t0 = clock64();
     return false;
@@ -274,7 +268,6 @@ __device__ __forceinline__ uint32_t ri_wait(const RiParams &P, uint32_t ring, ui
         if (ri_ld32(ri_base() + kRiDone)) return 0u;
         if (ri_try_feed(P, 1u)) continue;
         if (t0 == 0) t0 = clock64();
-        if (__any_sync(0xffffffffu, clock64() - t0 <= P.wait_cycles)) continue;
         if (ri_stalled(P, mark, t0)) {
             if ((threadIdx.x & 31u) == 0u) {
                 atomicOr(P.err, kPnErrTimeout);
@@ -382,10 +375,20 @@ __global__ void __launch_bounds__(kRiThreads, 1) pnfa_fp32_kernel(const __grid_c
         if (own) {   // the symbol after this one (bytes >= sigma are skipped)
             const uint8_t *p, *e;
             ri_ldp(rec + kRiRecP, p, e);
-            p += p < e;
+            bool found = p < e && nc < (uint32_t)P.sigma;
+            if (p < e) ++p;
+            if (!found && p < e) {
+                // (a byte at a time: reading lines here, or calling a function that does, costs registers
+                // and 3% of the time of every batch)
+                ri_add32(ri_base() + kRiBusy, 1u);
+                while (!found && p < e) {
+                    nc = __ldg(p++);
+                    found = nc < (uint32_t)P.sigma;
+                }
+                ri_add32(ri_base() + kRiBusy, 0xffffffffu);
+            }
+            ending = !found;
             ri_stp(rec + kRiRecP, p);
-            if (nc >= (uint32_t)P.sigma && p < e) nc = ri_next(rec, (uint32_t)P.sigma);
-            ending = nc >= (uint32_t)P.sigma;
         }
         const uint32_t ends = __ballot_sync(FULL, ending);
 #pragma unroll
