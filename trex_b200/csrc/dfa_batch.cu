@@ -1980,13 +1980,12 @@ static int dfa_set_run_ex(trex_dfa_set *set, const uint8_t *data, const int64_t 
     P.accept = accept;
     P.accept_i32 = accept_i32;
     // Small batches at the default item length: one launch (an explicit item length asks for the
-    // planned path). Measured, one launch against planned, us a call: 16 states, strings of 1024
-    // bytes, 16 KiB / 1 / 4 / 8 / 16 MiB: 14 / 15 / 19 / 27 / 37 against 86 / 78 / 101 / 116 / 117;
-    // log-normal strings (median 512): 15 / 33 / 44 / 62 / 83 against 125 / 126 / 147 / 162 / 188;
-    // 16 automata, strings of 64 bytes, 4 / 8 / 16 MiB: 33 / 58 / 108 against 69 / 74 / 84, so
-    // the limits lie at 8 MiB and as many strings as 64-byte ones make. Sets whose maps do not fit in
-    // shared memory are planned (64 automata of 64 states, 8000 strings of 1000 bytes: 220 read from
-    // L2 against 124).
+    // planned path). Measured, one launch against planned, us a call alone, 16 KiB / 1 / 4 / 8 MiB: 16
+    // states, strings of 1024 bytes, 27 / 29 / 35 / 45 against 98 / 91 / 94 / 96; 64 states, 34 / 36 / 49 / 57
+    // against 95 / 92 / 93 / 95; log-normal strings (median 512), 31 / 45 / 57 / 72 against 135 / 130 / 129 /
+    // 130; 16 automata, strings of 64 bytes, 22 / 30 / 51 / 79 against 65 / 71 / 74 / 80, so the limits
+    // lie at 8 MiB and as many strings as 64-byte ones make. Sets whose maps do not fit in shared memory
+    // are planned (64 automata of 64 states, 8000 strings of 1000 bytes: 220 read from L2 against 124).
     if (seg_len_in <= 0 && n <= kSmallStrings && walked <= kSmallBytes && set->tmap_bytes <= kSmallMapBytes) {
         P.fix_tm_bytes = (uint32_t)set->tmap_bytes;
         const int grid = (int)std::min<int64_t>(

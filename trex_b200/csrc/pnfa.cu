@@ -1074,8 +1074,9 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
             TREX_CHECK_LAUNCH();
             return TREX_OK;
         }
-        // alphabets whose tables fit on an SM: strings in rings by symbol (8192 strings x 512, 20
-        // symbols: 1.73 ms against 16.7); larger ones read every table through L1 and L2
+        // alphabets whose tables fit on an SM: strings in rings by symbol (20 symbols, 8192 strings x 512:
+        // 1.72 ms against 16.7; 64 x 512 0.59 against 2.3, one string of 4096 4.4 against 6.5); larger ones
+        // read every table through L1 and L2
         if (h->sigma <= kRiWarps) {
             RiParams S = ri_params(h, n_strings);
             S.data = data;
@@ -1103,7 +1104,9 @@ int trex_pnfa_run(trex_pnfa *h, int mode, const uint8_t *data, const int64_t *of
     }
     // Strings on TMEM lanes up to four symbols: at four, 262144 x 512 take 4.26 / 4.65 / 2.53 ms (BF16,
     // FP16, int8) there and 7.11 / 8.94 / 5.30 with lists by symbol; above, A's columns (32 a symbol)
-    // leave room for fewer tiles and B outgrows its 32 KB.
+    // leave room for fewer tiles and B outgrows its 32 KB. (The other side: below some ten thousand
+    // strings the lists spread them over more SMs, 512 x 2048 at four symbols 2.37 / 2.61 / 2.46 ms on
+    // lanes, 1.76 / 1.98 / 1.21 in lists; 32768 x 512 0.65 / 0.71 / 0.68 and 1.07 / 1.29 / 0.79.)
     if (h->sigma <= kLnMaxSigma) {
         const int k = mode == TREX_PNFA_FP16 ? 1 : mode == TREX_PNFA_BOOL8 ? 2 : mode == TREX_PNFA_BOOL ? 3 : 0;
         LnParams Q;

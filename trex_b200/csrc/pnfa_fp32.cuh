@@ -15,7 +15,7 @@
 // at every step, as there: the states are the same bits.
 //
 // 8192 strings x 512, 20 symbols: 16.7 -> 1.72 ms (0.26 -> 2.4 Gchar/s), the shared-memory pipe
-// 82% busy (80 wavefronts of table a group, 16 of states a string).
+// 83% busy (80 wavefronts of table a group, 16 of states a string).
 #pragma once
 
 namespace trex {
