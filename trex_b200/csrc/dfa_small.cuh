@@ -174,7 +174,8 @@ __device__ __noinline__ uint32_t small_piece(SmallMap map, uint32_t N, SmallView
                                              uint32_t start, int entry, uint64_t *s_map) {
     const uint32_t t = threadIdx.x, used = w1 - w0;
     const uint32_t k0 = min(w1, w0 + t), k1 = min(w1, k0 + 1u);
-    const uint32_t warm = (uint32_t)(warm_bytes((int)N, 224) / 32) * (t > 0u ? 1u : N <= 64u ? 2u : 4u);   // (a wrong entry costs the CTA a walk)
+    // (the piece's own entry warms up longer: a wrong one costs the whole CTA a walk)
+    const uint32_t warm = (uint32_t)(warm_bytes((int)N, 224) / 32) * (t > 0u ? 1u : N <= 64u ? 2u : 4u);
     const uint32_t first = entry >= 0 ? w0 : 0u;   // the first window whose entry state is known
     const uint32_t ks = k0 > first + warm ? k0 - warm : first;
     const uint32_t both = small_walk(map, v.lo, v.hi, v.w, k0 < k1 ? ks : k1, k1, k0,

@@ -18,8 +18,9 @@
 // append) with five warps a scheduler to hide it: 65536 strings x 2048 symbols, 20 symbols, BF16
 // take 7.03 ms, of which the MMAs' issue (2 cycles each on an SM) is 1.9 ms. tcgen05.mma needs 128
 // rows of A, two symbols' tables, throws half of every product away and brings it back through
-// TMEM: that form, with a step's strings sorted by symbol pair, took 20.65 ms. With mbarriers between the warps of a symbol instead of one barrier a step it took
-// 12.1 ms: a warp that polls takes issue slots and the shared-memory pipe from those that work.
+// TMEM: that form, with a step's strings sorted by symbol pair, took 20.65 ms. With mbarriers
+// between the warps of a symbol instead of one barrier a step it took 12.1 ms: a warp that polls takes
+// issue slots and the shared-memory pipe from those that work.
 #pragma once
 
 namespace trex {
